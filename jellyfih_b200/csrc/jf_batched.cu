@@ -20,15 +20,12 @@
 
 #include <utility>
 
-#include "jf_engine.h"
+#include "jf_chunk.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int kHaloLo = 1;  // window rows below the band (drift of one row)
-constexpr int kHaloHi = 3;  // rows above: the stencil's +2 plus one row of drift
-constexpr int kHalo = kHaloLo + kHaloHi;
 constexpr int kSortThreads = 256;
 constexpr int kScanThreads = 1024;
 // Per-lane cap of a cell's particles: a warp's cell loop runs as many
@@ -53,8 +50,6 @@ constexpr int kRowCost = 40;  // grid update of one row, in the cost model's uni
 // 2.3 % on the 32-instance batch against no weight).
 constexpr int kSolidCostHalves = 3;
 constexpr int kNoCap = 1 << 30;
-// CTA size of the TMEM variant of the chunk kernel (24 warps per SM)
-constexpr int kTmemThreads = 768;
 
 // Sort cell of a particle: (floor(X - 1/4), floor(Y - 1/4)) in grid units,
 // clamped at 0.  The stencil base trunc(X - 1/2) of a particle in sort cell k
@@ -98,21 +93,6 @@ struct ChunkArgs {
   unsigned long long* path;  // [register scatters, generic scatters, generic gathers, overflow]
 };
 
-// Shared-memory window of one CTA: grid rows [win0, win0 + WR) of its
-// instance: the updated velocity G as float2 pairs (one 64-bit load per node
-// in G2P), then planar accumulators (momentum Ax, Ay,
-// mass Am and, axisymmetric only, the hoop sum Ah).  Rows outside the window
-// are reached in the owner CTA's window.
-struct Window {
-  float2* G;
-  float *Ax, *Ay, *Am, *Ah;
-  int nx, win0;
-  int WR;  // rows of a plane (the largest band the sort may cut, plus the halo)
-  int VR;  // rows in use: this band's rows plus the halo; rows VR .. WR - 1 stay idle
-  int CS;
-  const int* brow;  // shared copy of the instance's band row starts (CS + 1)
-};
-
 // Distributed shared memory in explicit shared::cluster form: the address of
 // a local shared location in CTA `rank` of the cluster (mapa), and 32-bit
 // loads / reductions there, so that no generic pointer into another CTA's
@@ -132,264 +112,38 @@ __device__ __forceinline__ float2 dsmem_ld2(uint32_t a) {
   return v;
 }
 
-// Tensor memory (TMEM) variant of the cell lanes' node block.  With more than
-// 16 warps per SM the 48-float block no longer fits in registers beside one
-// particle's state, so between the particles of its cell a lane keeps the
-// block in TMEM: warp w of the CTA uses TMEM lanes 32 (w % 4) .. 32 (w % 4) + 31
-// (its threads' own lanes, the quadrant a warp may access) and the 48 columns
-// starting at 48 (w / 4) of the CTA's allocation.  Each access starts at a
-// multiple of its width in columns.  A load first waits for the thread's
-// earlier stores (tcgen05.wait::st; the second half needs none of its own,
-// see the cell loop) and waits for its data inside the same asm statement, so
-// its outputs cannot be read before they arrive.
-#define JF_TM_OUT16(b)                                                                                   \
-  "=r"(r[b + 0]), "=r"(r[b + 1]), "=r"(r[b + 2]), "=r"(r[b + 3]), "=r"(r[b + 4]), "=r"(r[b + 5]),        \
-      "=r"(r[b + 6]), "=r"(r[b + 7]), "=r"(r[b + 8]), "=r"(r[b + 9]), "=r"(r[b + 10]), "=r"(r[b + 11]), \
-      "=r"(r[b + 12]), "=r"(r[b + 13]), "=r"(r[b + 14]), "=r"(r[b + 15])
-#define JF_TM_IN16(b)                                                                                             \
-  "r"(r[b + 0]), "r"(r[b + 1]), "r"(r[b + 2]), "r"(r[b + 3]), "r"(r[b + 4]), "r"(r[b + 5]), "r"(r[b + 6]),      \
-      "r"(r[b + 7]), "r"(r[b + 8]), "r"(r[b + 9]), "r"(r[b + 10]), "r"(r[b + 11]), "r"(r[b + 12]), "r"(r[b + 13]), \
-      "r"(r[b + 14]), "r"(r[b + 15])
-#define JF_TM_OUT8(b) \
-  "=r"(r[b + 0]), "=r"(r[b + 1]), "=r"(r[b + 2]), "=r"(r[b + 3]), "=r"(r[b + 4]), "=r"(r[b + 5]), "=r"(r[b + 6]), "=r"(r[b + 7])
-#define JF_TM_IN8(b) \
-  "r"(r[b + 0]), "r"(r[b + 1]), "r"(r[b + 2]), "r"(r[b + 3]), "r"(r[b + 4]), "r"(r[b + 5]), "r"(r[b + 6]), "r"(r[b + 7])
+// The window of one CTA; rows outside it are reached in the owner CTA's window.
+struct Window : JfWindow {
+  int WR;  // rows of a plane (the largest band the sort may cut, plus the halo); rows VR .. WR - 1 stay idle
+  int CS;
+  const int* brow;  // shared copy of the instance's band row starts (CS + 1)
 
-// columns 0 .. 47 of the warp's block set to zero (a task's start)
-__device__ __forceinline__ void tm_zero48(uint32_t ta) {
-  const uint32_t z = 0u;
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3};\n\t"
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%1], {%3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3};\n\t"
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%2], {%3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3, %3};"
-      :
-      : "r"(ta), "r"(ta + 16u), "r"(ta + 32u), "r"(z)
-      : "memory");
-}
-// columns 0 .. 23 (block rows 0 and 1): 16 at 0, 8 at 16
-__device__ __forceinline__ void tm_load_rows01(uint32_t ta, float* acc) {
-  uint32_t r[24];
-  asm volatile(
-      "tcgen05.wait::st.sync.aligned;\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%24];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%25];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : JF_TM_OUT16(0), JF_TM_OUT8(16)
-      : "r"(ta), "r"(ta + 16u)
-      : "memory");
-#pragma unroll
-  for (int q = 0; q < 24; ++q) acc[q] = __uint_as_float(r[q]);
-}
-__device__ __forceinline__ void tm_store_rows01(uint32_t ta, const float* acc) {
-  uint32_t r[24];
-#pragma unroll
-  for (int q = 0; q < 24; ++q) r[q] = __float_as_uint(acc[q]);
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17};\n\t"
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%1], {%18, %19, %20, %21, %22, %23, %24, %25};"
-      :
-      : "r"(ta), "r"(ta + 16u), JF_TM_IN16(0), JF_TM_IN8(16)
-      : "memory");
-}
-// columns 24 .. 47 (block rows 2 and 3): 8 at 24, 16 at 32.  No wait for
-// earlier stores: the last store to these columns came before the wait of the
-// rows-0/1 load that precedes every use.
-__device__ __forceinline__ void tm_load_rows23(uint32_t ta, float* acc) {
-  uint32_t r[24];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%24];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23}, [%25];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : JF_TM_OUT8(0), JF_TM_OUT16(8)
-      : "r"(ta + 24u), "r"(ta + 32u)
-      : "memory");
-#pragma unroll
-  for (int q = 0; q < 24; ++q) acc[q] = __uint_as_float(r[q]);
-}
-__device__ __forceinline__ void tm_store_rows23(uint32_t ta, const float* acc) {
-  uint32_t r[24];
-#pragma unroll
-  for (int q = 0; q < 24; ++q) r[q] = __float_as_uint(acc[q]);
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%2, %3, %4, %5, %6, %7, %8, %9};\n\t"
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%1], {%10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25};"
-      :
-      : "r"(ta + 24u), "r"(ta + 32u), JF_TM_IN8(0), JF_TM_IN16(8)
-      : "memory");
-}
-#undef JF_TM_OUT16
-#undef JF_TM_IN16
-#undef JF_TM_OUT8
-#undef JF_TM_IN8
+  // the band (CTA of the cluster) that owns grid row j, and j's row in its window
+  __device__ __forceinline__ int owner_of(int j) const {
+    int o = 0;
+    while (o + 1 < CS && brow[o + 1] <= j) ++o;
+    return o;
+  }
+  __device__ __forceinline__ int owner_row(int j, int o) const { return j - (brow[o] - kHaloLo); }
 
-// the band (CTA of the cluster) that owns grid row j, and j's row in its window
-__device__ __forceinline__ int owner_of(const Window& w, int j) {
-  int o = 0;
-  while (o + 1 < w.CS && w.brow[o + 1] <= j) ++o;
-  return o;
-}
-__device__ __forceinline__ int owner_row(const Window& w, int j, int o) { return j - (w.brow[o] - kHaloLo); }
-
-__device__ __forceinline__ float2 gather_node(const Window& w, cg::cluster_group& cl, int i, int j) {
-  const int wr = j - w.win0;
-  if (wr >= 0 && wr < w.VR) {
-    const int n = wr * w.nx + i;
-    return w.G[n];
+  __device__ __forceinline__ float2 far_gather(int i, int j) const {
+    const int o = owner_of(j);
+    return dsmem_ld2(dsmem_addr(G + owner_row(j, o) * nx + i, o));
   }
-  const int o = owner_of(w, j);
-  const int n = owner_row(w, j, o) * w.nx + i;
-  return dsmem_ld2(dsmem_addr(w.G + n, o));
-}
-
-// Scatter of one particle's 9 stencil contributions with atomics, local when
-// the rows are in this CTA's window, else into the owner CTA's window.
-__device__ __forceinline__ void scatter_particle(const Window& w, cg::cluster_group& cl, const JfInst& I,
-                                                 const JfStencil& st, const JfScatter& sc) {
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const int row = st.by + j;
-    const int wr = row - w.win0;
-    if (wr >= 0 && wr < w.VR) {
-      const int rn = wr * w.nx + st.bx;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const float3 c = jf_node_contrib(I, st, sc, i, j);
-        atomicAdd(w.Ax + rn + i, c.x);
-        atomicAdd(w.Ay + rn + i, c.y);
-        atomicAdd(w.Am + rn + i, c.z);
-        if (I.axisym) atomicAdd(w.Ah + rn + i, jf_w(st, 0, i) * jf_w(st, 1, j) * sc.hoop);
-      }
-    } else {
-      const int o = owner_of(w, row);
-      const int rn = owner_row(w, row, o) * w.nx + st.bx;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const float3 c = jf_node_contrib(I, st, sc, i, j);
-        dsmem_add(dsmem_addr(w.Ax + rn + i, o), c.x);
-        dsmem_add(dsmem_addr(w.Ay + rn + i, o), c.y);
-        dsmem_add(dsmem_addr(w.Am + rn + i, o), c.z);
-        if (I.axisym) dsmem_add(dsmem_addr(w.Ah + rn + i, o), jf_w(st, 0, i) * jf_w(st, 1, j) * sc.hoop);
-      }
-    }
+  __device__ __forceinline__ void far_scatter(int i, int j, float3 c, float h, bool axisym) const {
+    const int o = owner_of(j);
+    const int n = owner_row(j, o) * nx + i;
+    dsmem_add(dsmem_addr(Ax + n, o), c.x);
+    dsmem_add(dsmem_addr(Ay + n, o), c.y);
+    dsmem_add(dsmem_addr(Am + n, o), c.z);
+    if (axisym) dsmem_add(dsmem_addr(Ah + n, o), h);
   }
-}
-
-// Adds a particle's 3x3 stencil into the lane's 4x4 node block, shifted by
-// (di, dj) = stencil base - (cell - 1), both 0 or 1.  Branch-free: the
-// weights are shifted into 4-wide vectors with zeros outside the stencil, so
-// lanes with different shifts run the same instructions.  Contributions are
-// formed separably, weight_x * (m v + A (x_i - x_p)) per column and then
-// weight_y per row, a re-association of mpm_sim.py:256-271 that moves results
-// by rounding only.
-__device__ __forceinline__ void accumulate_block(float* acc, const JfInst& I, const JfStencil& st,
-                                                 const JfScatter& sc, int di, int dj) {
-  const bool sx = di != 0, sy = dj != 0;
-  const float wx4[4] = {sx ? 0.0f : st.wx0, sx ? st.wx0 : st.wx1, sx ? st.wx1 : st.wx2, sx ? st.wx2 : 0.0f};
-  const float wy4[4] = {sy ? 0.0f : st.wy0, sy ? st.wy0 : st.wy1, sy ? st.wy1 : st.wy2, sy ? st.wy2 : 0.0f};
-  // node offsets from the particle: (I - di - fx0) dx; di + fx0 is exact
-  const float ex = (float)di + st.fx0, ey = (float)dj + st.fx1;
-  float P[4], Q0[4], Q1[4], Pm[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float d0 = ((float)i - ex) * I.dx;
-    P[i] = wx4[i];
-    Q0[i] = wx4[i] * (sc.mv0 + sc.af00 * d0);
-    Q1[i] = wx4[i] * (sc.mv1 + sc.af10 * d0);
-    Pm[i] = wx4[i] * sc.mass;
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float d1 = ((float)j - ey) * I.dx;
-    const float r0 = sc.af01 * d1, r1 = sc.af11 * d1;
-    const float wj = wy4[j];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int q = (j * 4 + i) * 3;
-      acc[q + 0] += wj * (Q0[i] + P[i] * r0);
-      acc[q + 1] += wj * (Q1[i] + P[i] * r1);
-      acc[q + 2] += wj * Pm[i];
-    }
-  }
-}
-
-// accumulate_block restricted to block rows J0 and J0 + 1, whose 24 floats
-// `acc` holds (the TMEM variant adds a particle half a block at a time).
-template <int J0>
-__device__ __forceinline__ void accumulate_rows(float* acc, const JfInst& I, const JfStencil& st,
-                                                const JfScatter& sc, int di, int dj) {
-  const bool sx = di != 0, sy = dj != 0;
-  const float wx4[4] = {sx ? 0.0f : st.wx0, sx ? st.wx0 : st.wx1, sx ? st.wx1 : st.wx2, sx ? st.wx2 : 0.0f};
-  const float wy4[4] = {sy ? 0.0f : st.wy0, sy ? st.wy0 : st.wy1, sy ? st.wy1 : st.wy2, sy ? st.wy2 : 0.0f};
-  const float ex = (float)di + st.fx0, ey = (float)dj + st.fx1;
-  float P[4], Q0[4], Q1[4], Pm[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float d0 = ((float)i - ex) * I.dx;
-    P[i] = wx4[i];
-    Q0[i] = wx4[i] * (sc.mv0 + sc.af00 * d0);
-    Q1[i] = wx4[i] * (sc.mv1 + sc.af10 * d0);
-    Pm[i] = wx4[i] * sc.mass;
-  }
-#pragma unroll
-  for (int jj = 0; jj < 2; ++jj) {
-    const int j = J0 + jj;
-    const float d1 = ((float)j - ey) * I.dx;
-    const float r0 = sc.af01 * d1, r1 = sc.af11 * d1;
-    const float wj = wy4[j];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int q = (jj * 4 + i) * 3;
-      acc[q + 0] += wj * (Q0[i] + P[i] * r0);
-      acc[q + 1] += wj * (Q1[i] + P[i] * r1);
-      acc[q + 2] += wj * Pm[i];
-    }
-  }
-}
-
-// Writes a warp's 4x4 node blocks into the window.  Lane l owns cell column
-// cx = seg0 + l and covers node columns cx-1 .. cx+2; node column cx collects
-// block column 1 of lane l, 0 of lane l+1, 2 of lane l-1 and 3 of lane l-2,
-// so each lane issues one atomic per (row, component).  Lane 0 also writes
-// column seg0-1, lane 31 columns seg0+32 and seg0+33.
-// `acc` holds block rows J0 .. J0 + NJ - 1 (the TMEM variant flushes two rows
-// at a time).
-template <int J0 = 0, int NJ = 4>
-__device__ __forceinline__ void flush_block(const float* acc, const Window& w, int lane, int cx, int cy,
-                                            int seg0, int nx) {
-  const unsigned full = 0xffffffffu;
-#pragma unroll
-  for (int J = J0; J < J0 + NJ; ++J) {
-    const int rowo = (cy - 1 + J - w.win0) * nx;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      float* A = q == 0 ? w.Ax : (q == 1 ? w.Ay : w.Am);
-      const float a0 = acc[((J - J0) * 4 + 0) * 3 + q];
-      const float a1 = acc[((J - J0) * 4 + 1) * 3 + q];
-      const float a2 = acc[((J - J0) * 4 + 2) * 3 + q];
-      const float a3 = acc[((J - J0) * 4 + 3) * 3 + q];
-      const float from_right = __shfl_down_sync(full, a0, 1);
-      const float from_left = __shfl_up_sync(full, a2, 1);
-      const float from_left2 = __shfl_up_sync(full, a3, 2);
-      const float a3_l30 = __shfl_sync(full, a3, 30);
-      float col = a1;
-      if (lane <= 30) col += from_right;
-      if (lane >= 1) col += from_left;
-      if (lane >= 2) col += from_left2;
-      if (cx < nx && col != 0.0f) atomicAdd(A + rowo + cx, col);
-      if (lane == 0 && seg0 >= 1 && a0 != 0.0f) atomicAdd(A + rowo + seg0 - 1, a0);
-      if (lane == 31) {
-        const float e32 = a2 + a3_l30;
-        if (seg0 + 32 < nx && e32 != 0.0f) atomicAdd(A + rowo + seg0 + 32, e32);
-        if (seg0 + 33 < nx && a3 != 0.0f) atomicAdd(A + rowo + seg0 + 33, a3);
-      }
-    }
-  }
-}
+};
 
 // kTmem: the node blocks live in TMEM (launched with 544 .. 768 threads, 80
 // registers at 768); otherwise in registers (up to 512 threads, 128 registers).
 template <bool kTmem>
-__global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(ChunkArgs a) {
+__global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(const __grid_constant__ ChunkArgs a) {
   extern __shared__ float4 smem4[];
   float* sm = reinterpret_cast<float*>(smem4);
   // per-substep values, double-buffered so that substep s + 1's are set
@@ -406,7 +160,6 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
 
   const JfInst I = a.inst[m];
   const JfParams P = a.params[m];
-  const JfMaterials mats = a.mats;
   const int nx = I.nx, ny = I.ny;
   __shared__ int s_brow[kMaxCluster + 1];
   if (threadIdx.x <= CS) s_brow[threadIdx.x] = a.brow[m * (CS + 1) + threadIdx.x];
@@ -432,12 +185,8 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
   const int lane = tid & 31, warp = tid >> 5, n_warps = nth >> 5;
   const int cells = nx * ny;
   const int32_t* cstart = a.cell_start + (int64_t)m * a.stride;
-  const int64_t p0 = I.p_off;
-  // this instance's particle arrays, indexed by position within the instance
-  float4* __restrict__ xv_m = a.xv + p0;
-  float4* __restrict__ C_m = a.C + p0;
-  float4* __restrict__ F_m = a.F + p0;
-  const int32_t* __restrict__ mat_m = a.mat + p0;
+  const int p0 = (int)I.p_off;
+  const JfEnv<ChunkArgs> E{I, a, P.payload_density, a.do_glow != 0};
 
   for (int n = tid; n < n_planes * WN; n += nth) sm[n] = 0.0f;
   // path counters of the CTA: register-block scatters, per-particle (generic)
@@ -453,14 +202,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
   if constexpr (kTmem) {
     const int per_quad = (n_warps + 3) >> 2;
     while (tm_cols < (uint32_t)(48 * per_quad)) tm_cols <<= 1;
-    __syncwarp();
-    if (warp == 0) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                       (uint32_t)__cvta_generic_to_shared(&s_tmem)),
-                   "r"(tm_cols)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    if (warp == 0) tm_alloc(&s_tmem, tm_cols);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   cluster.sync();
@@ -469,39 +211,6 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
     tm_base = s_tmem;
     ta = tm_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(48 * (warp >> 2));
   }
-
-  // G2P of the previous substep, then P2G of this one, for a particle that
-  // is not handled by a cell lane (generic gathers and scatters).
-  auto particle_generic = [&](int64_t g, bool do_g2p, bool do_p2g, float pressure) {
-    const float4 xv = a.xv[g];
-    float4 C = a.C[g];
-    const int mt = a.mat[g];
-    float2 x = make_float2(xv.x, xv.y), v = make_float2(xv.z, xv.w);
-    float jp = 1.0f;
-    if (mt == 2 || a.do_glow) jp = a.Jp[g];
-    if (do_g2p) {
-      jf_g2p_particle(I, x, v, C, [&](int ni, int nj) { return gather_node(w, cluster, ni, nj); });
-      if (a.do_glow) a.glow[g] = jf_glow(a.glow[g], jp);
-      nonfinite |= !(isfinite(x.x) && isfinite(x.y) && isfinite(v.x) && isfinite(v.y));
-      a.xv[g] = make_float4(x.x, x.y, v.x, v.y);
-      if (!do_p2g) a.C[g] = C;  // stored when no later pass of the chunk recomputes it (see the cell loop)
-    }
-    if (do_p2g) {
-      JfStencil st;
-      if (jf_stencil(I, x, st)) {
-        float4 F = a.F[g];
-        const float2 fb = (mt == 3) ? a.fiber[g] : make_float2(0.0f, 1.0f);
-        JfScatter sc;
-        jf_p2g_particle(I, mats, mt, v, C, F, jp, fb, pressure, P.payload_density, sc, x.x,
-                        I.axisym ? a.rref[g] : 1.0f);
-        a.F[g] = F;
-        if (mt == 2) a.Jp[g] = jp;
-        scatter_particle(w, cluster, I, st, sc);
-      } else if (do_g2p) {
-        a.C[g] = C;  // out of range: the next G2P keeps this C
-      }
-    }
-  };
 
   // tasks: groups of 32 generic particles (this band's overflow list, then,
   // in the last band, live particles outside every stencil range), then the
@@ -543,173 +252,28 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
     // cells of the band: a warp takes 32 consecutive cells of one row; warps
     // claim row segments from a shared counter so that they finish together
     for (int task_id = warp; task_id < n_tasks;) {
-      if (task_id < n_gen_tasks) {
+      const bool generic = task_id < n_gen_tasks;
+      int beg = 0, end = 0, cy = 0, seg0 = 0;  // the lane's particles, as engine positions
+      if (generic) {
         const int e = task_id + lane * n_gen_tasks;
         if (e < n_generic_all) {
           const bool over = e < n_ov;
-          particle_generic(p0 + (over ? ov[e] : oor_beg + e - n_ov), do_g2p, do_p2g, pressure);
+          beg = p0 + (over ? ov[e] : oor_beg + e - n_ov);
+          end = beg + 1;
           atomicAdd(&s_path[over ? 3 : 1], 1u);
         }
-        int nt = 0;
-        if (lane == 0) nt = atomicAdd(next_task, 1);
-        task_id = __shfl_sync(0xffffffffu, nt, 0);
-        continue;
-      }
-      const int task = task_id - n_gen_tasks;
-      const int cy = row0 + task / segs;
-      const int seg0 = (task % segs) << 5;
-      const int cx = seg0 + lane;
-      int beg = 0, end = 0;
-      if (cx < nx) {
-        const int c = cy * nx + cx;
-        beg = cstart[c];
-        end = min(cstart[c + 1], beg + cap);  // the rest of the cell is overflow
-      }
-      // G2P then P2G of particle k of this lane's cell (nxv / nmt: its
-      // prefetched position-velocity and material, replaced by particle
-      // k + 1's); returns true when its stencil lies in the lane's 4x4 node
-      // block (columns cx-1 .. cx+2, rows cy-1 .. cy+2), with the stencil,
-      // the scatter terms and the block offset for the caller to add
-      auto cell_particle = [&](int k, float4& nxv, int& nmt, JfStencil& st, JfScatter& sc, int& di,
-                               int& dj) -> bool {
-        const float4 xv = nxv;
-        const int mt = nmt;
-        float4 F = F_m[k];  // first used by P2G, after the gather
-        if (k + 1 < end) {  // next particle of this cell, loaded while this one computes
-          nxv = xv_m[k + 1];
-          nmt = mat_m[k + 1];
-        }
-        float2 x = make_float2(xv.x, xv.y), v = make_float2(xv.z, xv.w);
-        float jp = 1.0f;
-        if (mt == 2 || a.do_glow) jp = a.Jp[p0 + k];
-        // G2P replaces v and C from the grid (mpm_sim.py:315-327); the stored
-        // C is read only where G2P does not run
-        float4 C;
-        if (do_g2p) {
-          JfStencil gs;
-          if (!jf_stencil(I, x, gs)) {
-            C = C_m[k];
-          } else {
-            const int wr0 = gs.by - w.win0;
-            if (wr0 >= 0 && wr0 + 2 < w.VR) {
-              const int wb = wr0 * nx + gs.bx;
-              jf_g2p_apic(I, gs, v, C, [&](int i, int j) {
-                const int n = wb + j * nx + i;
-                return w.G[n];
-              });
-            } else {
-              atomicAdd(&s_path[2], 1u);
-              jf_g2p_apic(I, gs, v, C,
-                          [&](int i, int j) { return gather_node(w, cluster, gs.bx + i, gs.by + j); });
-            }
-          }
-          jf_g2p_advect(I, x, v);
-          if (a.do_glow) a.glow[p0 + k] = jf_glow(a.glow[p0 + k], jp);
-          nonfinite |= !(isfinite(x.x) && isfinite(x.y) && isfinite(v.x) && isfinite(v.y));
-          xv_m[k] = make_float4(x.x, x.y, v.x, v.y);
-          // this pass's P2G takes C from registers and the next pass's G2P
-          // recomputes it, so C is stored only by the chunk's last pass and
-          // where the particle leaves the stencil range (P2G below)
-          if (!do_p2g) C_m[k] = C;
-        } else {
-          C = C_m[k];
-        }
-        if (!do_p2g) return false;
-        if (!jf_stencil(I, x, st)) {
-          if (do_g2p) C_m[k] = C;  // out of range: the next G2P keeps this C
-          return false;
-        }
-        const float2 fb = (mt == 3) ? a.fiber[p0 + k] : make_float2(0.0f, 1.0f);
-        jf_p2g_particle(I, mats, mt, v, C, F, jp, fb, pressure, P.payload_density, sc, x.x,
-                        I.axisym ? a.rref[p0 + k] : 1.0f);
-        F_m[k] = F;
-        if (mt == 2) a.Jp[p0 + k] = jp;
-        di = st.bx - (cx - 1);
-        dj = st.by - (cy - 1);
-        if ((unsigned)di < 2u && (unsigned)dj < 2u) {
-          if (I.axisym) {  // the hoop sum goes straight to the window (rows in it)
-            const int hb = (st.by - w.win0) * nx + st.bx;
-#pragma unroll
-            for (int jj = 0; jj < 3; ++jj)
-#pragma unroll
-              for (int ii = 0; ii < 3; ++ii)
-                atomicAdd(w.Ah + hb + jj * nx + ii, jf_w(st, 0, ii) * jf_w(st, 1, jj) * sc.hoop);
-          }
-          return true;
-        }
-        atomicAdd(&s_path[1], 1u);
-        scatter_particle(w, cluster, I, st, sc);
-        return false;
-      };
-      float4 nxv;
-      int nmt = -1;
-      if (beg < end) {
-        nxv = xv_m[beg];
-        nmt = mat_m[beg];
-      }
-      if constexpr (!kTmem) {
-        // the lane's cell runs as a loop of its own length; the block stays in registers
-        unsigned n_block = 0;
-        float acc[48];
-#pragma unroll
-        for (int q = 0; q < 48; ++q) acc[q] = 0.0f;
-        for (int k = beg; k < end; ++k) {
-          JfStencil st;
-          JfScatter sc;
-          int di, dj;
-          if (cell_particle(k, nxv, nmt, st, sc, di, dj)) {
-            accumulate_block(acc, I, st, sc, di, dj);
-            ++n_block;
-          }
-        }
-        __syncwarp();
-        if (do_p2g) {
-          flush_block(acc, w, lane, cx, cy, seg0, nx);
-          const unsigned nb = __reduce_add_sync(0xffffffffu, n_block);
-          if (lane == 0 && nb) atomicAdd(&s_path[0], nb);
-        }
       } else {
-        // the warp steps its cells' particles together (the TMEM accesses are
-        // warp-wide) for as many iterations as its fullest cell; the block of
-        // each lane is loaded from TMEM, added to and stored back, two rows at
-        // a time, once per iteration in which some lane's particle adds to it
-        const int iters = (int)__reduce_max_sync(0xffffffffu, (unsigned)(end - beg));
-        unsigned n_block = 0;  // the same in every lane of the warp
-        __syncwarp();
-        if (do_p2g) tm_zero48(ta);
-        for (int it = 0; it < iters; ++it) {
-          const int k = beg + it;
-          JfStencil st;
-          JfScatter sc;
-          int di = 0, dj = 0;
-          const bool blk = k < end && cell_particle(k, nxv, nmt, st, sc, di, dj);
-          if (do_p2g) {
-            const unsigned bm = __ballot_sync(0xffffffffu, blk);
-            if (bm) {
-              n_block += (unsigned)__popc(bm);
-              float half[24];
-              tm_load_rows01(ta, half);
-              if (blk) accumulate_rows<0>(half, I, st, sc, di, dj);
-              __syncwarp();
-              tm_store_rows01(ta, half);
-              tm_load_rows23(ta, half);
-              if (blk) accumulate_rows<2>(half, I, st, sc, di, dj);
-              __syncwarp();
-              tm_store_rows23(ta, half);
-            }
-          }
-        }
-        __syncwarp();
-        if (do_p2g) {
-          // the last store to columns 24 .. 47 precedes the wait of the first load
-          float half[24];
-          tm_load_rows01(ta, half);
-          flush_block<0, 2>(half, w, lane, cx, cy, seg0, nx);
-          tm_load_rows23(ta, half);
-          flush_block<2, 2>(half, w, lane, cx, cy, seg0, nx);
-          if (lane == 0 && n_block) atomicAdd(&s_path[0], n_block);
+        const int task = task_id - n_gen_tasks;
+        cy = row0 + task / segs;
+        seg0 = (task % segs) << 5;
+        if (seg0 + lane < nx) {
+          const int c = cy * nx + seg0 + lane;
+          beg = p0 + cstart[c];
+          end = p0 + cstart[c + 1];
+          if (end - beg > cap) end = beg + cap;  // the rest of the cell is overflow
         }
       }
+      run_task<kTmem>(E, w, !generic, beg, end, cy, seg0, ta, do_g2p, do_p2g, pressure, s_path, nonfinite);
       int nt = 0;
       if (lane == 0) nt = atomicAdd(next_task, 1);
       task_id = __shfl_sync(0xffffffffu, nt, 0);
@@ -727,8 +291,8 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
         const float vx = w.Ax[n], vy = w.Ay[n], vm = w.Am[n];
         const float vh = I.axisym ? w.Ah[n] : 0.0f;
         if (vx != 0.0f || vy != 0.0f || vm != 0.0f || vh != 0.0f) {
-          const int o = owner_of(w, j);
-          const int rn = owner_row(w, j, o) * nx + (n - wr * nx);
+          const int o = w.owner_of(j);
+          const int rn = w.owner_row(j, o) * nx + (n - wr * nx);
           dsmem_add(dsmem_addr(w.Ax + rn, o), vx);
           dsmem_add(dsmem_addr(w.Ay + rn, o), vy);
           dsmem_add(dsmem_addr(w.Am + rn, o), vm);
@@ -776,8 +340,8 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
         const int j = w.win0 + wr;
         if (j < 0 || j >= ny) continue;
         const int n = wr * nx + (q - h * nx);
-        const int o = owner_of(w, j);
-        const int rn = owner_row(w, j, o) * nx + (n - wr * nx);
+        const int o = w.owner_of(j);
+        const int rn = w.owner_row(j, o) * nx + (n - wr * nx);
         w.G[n] = dsmem_ld2(dsmem_addr(w.G + rn, o));
       }
       t = t + a.dt;
@@ -796,8 +360,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) chunk_kernel(Ch
   if constexpr (kTmem) {
     if (warp == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(tm_cols)
-                   : "memory");
+      tm_free(tm_base, tm_cols);
     }
   }
   if (a.path && tid < 4 && s_path[tid]) atomicAdd(a.path + tid, (unsigned long long)s_path[tid]);
@@ -1097,7 +660,7 @@ cudaError_t jf_batched_sort(jf_engine* e) {
   return cudaSuccess;
 }
 
-static cudaError_t launch_chunk(jf_engine* e, int K) {
+static cudaError_t launch_clusters(jf_engine* e, int K) {
   ChunkArgs a;
   a.inst = e->d_inst;
   a.params = e->d_params;
@@ -1139,15 +702,19 @@ static cudaError_t launch_chunk(jf_engine* e, int K) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  e->launches += 1;
+  return e->block_threads > 512 ? cudaLaunchKernelEx(&cfg, chunk_kernel<true>, a)
+                                : cudaLaunchKernelEx(&cfg, chunk_kernel<false>, a);
+}
+
+static cudaError_t launch_chunk(jf_engine* e, int K) {
   cudaError_t err;
   {
     JfTimed timed(e, false, e->capturing);
-    err = e->block_threads > 512 ? cudaLaunchKernelEx(&cfg, chunk_kernel<true>, a)
-                                 : cudaLaunchKernelEx(&cfg, chunk_kernel<false>, a);
+    err = launch_clusters(e, K);
   }
-  e->launches += 1;
   if (err != cudaSuccess) return err;
-  if (a.do_glow) {
+  if (e->flags & JF_FLAG_GLOW) {
     dead_glow_kernel<<<dim3(16, e->M), 256, 0, e->stream>>>(e->d_inst, e->d_band, e->cluster, e->p.mat,
                                                            e->p.Jp, e->p.glow, K);
     e->launches += 1;
@@ -1213,6 +780,7 @@ static cudaError_t capture_pair(jf_engine* e, int K) {
   cudaError_t e2 = (e1 == cudaSuccess) ? chunk_with_sort(e, K) : e1;
   e->capturing = false;
   err = cudaStreamEndCapture(e->stream, &graph);
+  e->graph_launches = e->launches - launches;
   e->launches = launches;  // nothing ran yet
   if (e2 != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
@@ -1224,7 +792,6 @@ static cudaError_t capture_pair(jf_engine* e, int K) {
   if (err != cudaSuccess) return err;
   e->graph_K = K;
   e->graph_p = e->p.xv;
-  e->graph_launches = 2 * (e->max_slots > 0 ? 5 : 3) + ((e->flags & JF_FLAG_GLOW) ? 2 : 0);
   return cudaSuccess;
 }
 
