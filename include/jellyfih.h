@@ -70,10 +70,15 @@ typedef struct {
   int32_t resort_interval;              /* batched: substeps between re-sorts, 0 = 64 */
   int32_t block_threads;                /* batched: threads per CTA (multiple of 32, <= 768); above
                                            512 the cell lanes keep their node blocks in tensor
-                                           memory (TMEM), up to 512 in registers.  0 = 768 when the
-                                           tallest instance's bands hold >= 32 rows
+                                           memory (TMEM), up to 512 in registers.  0 = automatic:
+                                           512 for spans; for clusters 768 when the tallest
+                                           instance's bands hold >= 32 rows
                                            (ceil(n_grid_y / cluster size)), else 512 */
-  int32_t cluster_size;                 /* batched: CTAs per instance (1..16), 0 = automatic */
+  int32_t cluster_size;                 /* batched: one cluster of this many CTAs (1..16) per
+                                           instance.  0 = automatic: the grid rows of the whole
+                                           batch cut into one span of equal cost per SM, or
+                                           clusters where the batch does not suit that (instances
+                                           of different n_grid, n_grid_y > 1024) */
   int32_t cell_cap;                     /* batched: particles a cell lane accumulates per substep;
                                            the rest of the cell goes through per-particle atomics.
                                            0 = chosen per instance at every re-sort, >= 16 = no cap */
@@ -294,9 +299,11 @@ int jf_clear_error_flags(jf_engine* e);
  * (per-particle atomics).  All zero on the plain path. */
 int jf_path_counts(jf_engine* e, int64_t* out, int32_t reset);
 
-/* The batched launch layout the engine chose: CTAs per instance (cluster
- * size) and threads per CTA.  Either pointer may be NULL.  No counterpart in
- * the reference (its launch layout is Taichi's). */
+/* The cluster layout of the batch: CTAs per instance (cluster size) and threads
+ * per CTA, as configured or as its shape gives them.  A batch that runs as
+ * spans (jf_config.cluster_size 0) uses neither unless block_threads was set.
+ * Either pointer may be NULL.  No counterpart in the reference (its launch
+ * layout is Taichi's). */
 int jf_get_layout(const jf_engine* e, int32_t* cluster_size, int32_t* block_threads);
 
 /* Largest grid, in nodes (n_grid * n_grid_y), jf_substep_noalloc accepts. */

@@ -1,5 +1,7 @@
-// Batched path: every instance advances in one persistent launch per chunk
-// of substeps.  Instance m is owned by one thread-block cluster of CS CTAs
+// Batched path, clusters (for a cluster size asked for, and batches that do not
+// suit the spans of jf_span.cu), and the sort and chunk loop of both layouts:
+// every instance advances in one persistent launch per chunk of substeps.
+// Instance m is owned by one thread-block cluster of CS CTAs
 // (clusters take instances in descending live count); CTA r of the cluster
 // owns a band of grid rows of that instance — the bands are cut at each
 // re-sort so that the CTAs carry equal work — and keeps them, plus a halo, in
@@ -644,6 +646,14 @@ cudaError_t jf_batched_sort(jf_engine* e) {
     sort_keys_kernel<<<grid, kSortThreads, 0, e->stream>>>(e->d_inst, e->p.xv, e->p.mat, e->d_keys,
                                                           e->d_rank, e->d_counts, stride, e->d_solid);
   }
+  if (e->span) {
+    err = jf_span_sort(e);
+    e->launches += (e->max_slots > 0) ? 4 : 2;
+    if (err != cudaSuccess) return err;
+    std::swap(e->p, e->q);
+    e->sorted = true;
+    return cudaSuccess;
+  }
   sort_scan_kernel<<<e->M, kScanThreads, 0, e->stream>>>(e->d_inst, e->d_counts, stride, e->d_band,
                                                          e->d_brow, e->d_cap, e->d_ovband, e->d_ovcur,
                                                          e->cluster, e->cell_cap, e->d_solid);
@@ -711,7 +721,7 @@ static cudaError_t launch_chunk(jf_engine* e, int K) {
   cudaError_t err;
   {
     JfTimed timed(e, false, e->capturing);
-    err = launch_clusters(e, K);
+    err = e->span ? jf_span_launch(e, K) : launch_clusters(e, K);
   }
   if (err != cudaSuccess) return err;
   if (e->flags & JF_FLAG_GLOW) {

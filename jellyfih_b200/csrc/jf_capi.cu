@@ -302,7 +302,7 @@ int jf_create(const jf_config* cfg, jf_engine** out) {
            (ny_max + e->cluster * 2 - 1) / (e->cluster * 2) >= 8)
       e->cluster *= 2;
   }
-  // CTA size: 24 warps (node blocks in TMEM) when a band has rows enough to
+  // CTA size of the clusters: 24 warps (node blocks in TMEM) when a band has rows enough to
   // keep them busy to the end of a pass (32 rows = 128 cell tasks of 32 cells
   // on 128^2), else 16 warps (node blocks in registers): measured, 32-row
   // bands run 4 % faster at 768 threads, 16-row bands 16 % slower
@@ -410,6 +410,9 @@ int jf_create(const jf_config* cfg, jf_engine** out) {
     jf_batched_max_active_clusters(e, e->cluster, &active);
     if (active == 0)
       return bail(JF_ERR_UNSUPPORTED, "clusters of " + std::to_string(e->cluster) + " CTAs cannot be scheduled");
+    // without a cluster size asked for, the batch runs as one span of rows per SM where it can
+    if (cfg->cluster_size == 0 && (err = jf_span_setup(e, cfg->block_threads)) != cudaSuccess)
+      return bail(JF_ERR_CUDA, std::string("span set-up: ") + cudaGetErrorString(err));
   }
   if (cudaMemcpy(e->d_inst, e->inst.data(), sizeof(JfInst) * e->M, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(e->d_grid, 0, sizeof(float4) * std::max<int64_t>(g_off, 1)) != cudaSuccess ||
@@ -436,6 +439,7 @@ int jf_destroy(jf_engine* e) {
   cudaSetDevice(e->device);
   if (e->stream) cudaStreamSynchronize(e->stream);
   jf_grad_free(e);
+  jf_span_free(e);
   free_particles(e->p);
   free_particles(e->q);
   cudaFree(e->d_inst); cudaFree(e->d_params); cudaFree(e->d_keys); cudaFree(e->d_counts);
@@ -620,6 +624,9 @@ static int nonfinite_status(jf_engine* e, const std::vector<int32_t>& flags) {
   std::string which;
   int n = 0;
   for (int m = 0; m < e->M; ++m) {
+    if (flags[m] & kJfErrAbort)
+      return fail(e, JF_ERR_CUDA, "the step of instance " + std::to_string(m) +
+                                      " gave up waiting for another thread block; its state is not to be used");
     if (!flags[m]) continue;
     if (n < 8) which += (n ? ", " : "") + std::to_string(m);
     ++n;

@@ -1,6 +1,6 @@
-// What the batched chunk kernel is made of: the shared-memory window's layout,
+// What the two batched chunk kernels share: the shared-memory window's layout,
 // the cell lanes' node blocks (in registers or in tensor memory) and the tasks
-// of one pass over an instance's particles, written for any window
+// of one pass over an instance's particles, written for either kernel's window
 // type.  A window W has the fields G, Ax, Ay, Am, Ah, nx, win0 and VR of
 // JfWindow, and two members for grid rows outside it: far_gather(i, j), the
 // updated velocity of a node, and far_scatter(i, j, c, h), which adds a

@@ -27,6 +27,9 @@ struct JfParticles {
 };
 
 struct JfGrad;
+struct JfSpan;
+// Error flag of an instance whose chunk gave up waiting for another CTA.
+constexpr int32_t kJfErrAbort = 256;
 // Grids up to this many rows get bands balanced by per-row cost at each
 // re-sort (taller grids keep equal bands).
 constexpr int kJfMaxBandRows = 1024;
@@ -95,6 +98,7 @@ struct jf_engine {
   int64_t launches = 0;            // kernels launched by this engine
   std::string err;
 
+  JfSpan* span = nullptr;          // batched path: spans over all SMs (jf_span.cu); null: one cluster per instance
   JfGrad* grad = nullptr;          // differentiable rollout buffers (jf_grad.cu)
   // headless renderer (jf_render.cu)
   float4* d_frame = nullptr;       // frame_res^2 pixels (r, g, b, unused), row py = frame row
@@ -135,6 +139,14 @@ cudaError_t jf_plain_step(jf_engine* e, int64_t n_steps);
 cudaError_t jf_batched_step(jf_engine* e, int64_t n_steps);
 cudaError_t jf_batched_sort(jf_engine* e);
 size_t jf_batched_smem_bytes(const jf_engine* e);
+
+// Spans (jf_span.cu): the batched path's layout when the caller asks for no
+// cluster size.
+// threads: CTA size asked for, 0 = automatic.
+cudaError_t jf_span_setup(jf_engine* e, int threads);
+cudaError_t jf_span_sort(jf_engine* e);
+cudaError_t jf_span_launch(jf_engine* e, int K);
+void jf_span_free(jf_engine* e);
 
 // Episode helpers (jf_run_episode): load every instance from slot-ordered
 // staging, and the (M, 5) rows from before / after CoM sums, on the device.

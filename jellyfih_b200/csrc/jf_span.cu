@@ -1,0 +1,1017 @@
+// Batched path, spans: the grid rows of all instances, one instance after the
+// other, are cut into one contiguous span of about equal cost per SM at every
+// re-sort, and one cooperative launch per chunk of substeps advances them all,
+// one CTA per span.  A CTA owns the bands of rows (one per instance that its
+// span touches) and keeps them, plus a halo, in shared memory for the whole
+// chunk.
+//
+// Why spans and not one thread-block cluster per instance: clusters are placed
+// per GPC, so that at one CTA per SM only 33 clusters of 4, 15 of 8 or 7 of 16
+// fit a B200 (cudaOccupancyMaxActiveClusters): 32 instances use 128 of the 148
+// SMs, and 16 instances on clusters of 8 or 8 on clusters of 16 take two
+// waves.  Spans use every SM at every batch size, and an instance may share an
+// SM with the next one.
+//
+// One pass over a CTA's particles fuses G2P of substep s-1 with P2G of substep
+// s (mpm_sim.py:312-333 then :168-271).  Neighbouring bands of an instance
+// overlap in the four rows around their cut (the stencil's reach plus one row
+// of drift either way).  After a pass each side writes its partial sums of
+// those rows to global memory, the instance's CTAs meet at a counter, and each
+// side adds the other's sums and updates the rows for itself: the same two
+// terms, so the same bits, and one meeting per substep.  The rows between are
+// updated while the counters travel.
+//
+// A particle whose stencil has drifted out of its CTA's window (more than a
+// row since the last re-sort) adds to a spill grid in global memory and raises
+// the instance's drift flag of that substep; the instance's CTAs then add the
+// spill to their rows, publish their updated rows and meet a second time, so
+// that the particle can gather them in the next pass.  The result does not
+// depend on the re-sort interval.
+//
+// Every wait counts its polls and gives up after kSpinLimit: the CTA raises
+// the abort flag, which ends the waits of the others, frees its tensor memory
+// and returns, and the instance's error flag kErrAbort is set.
+#include <algorithm>
+#include <utility>
+#include <vector>
+
+#include "jf_chunk.cuh"
+
+namespace {
+
+constexpr int kMaxSeg = 8;        // bands of one CTA
+constexpr int kMinRows = 4;       // rows of a band: the overlaps of its two cuts stay apart
+constexpr int kOverlap = 4;       // rows around a cut that both sides hold
+// CTA size where the caller asks for none: 16 warps with the node blocks in
+// registers beat 24 with the blocks in TMEM at every batch size since the
+// packed arithmetic (us per substep, 80K-slot tanks on 128^2: 32 instances 81.9
+// against 86.2, 16: 45.8 against 48.7).
+constexpr int kSpanThreads = 512;
+constexpr int kScanThreads = 1024;
+constexpr int kMoveThreads = 256;
+// The cell cap and the row costs follow the same model as the cluster path's
+// sort (jf_batched.cu): 128 per warp iteration, 6 per overflow particle, 40
+// for a row's grid update, 1.5 per non-water particle.
+constexpr int kCapCandidates = 16;
+constexpr int kNoCap = 1 << 30;
+constexpr int kRowCost = 40;
+constexpr int kSolidCostHalves = 3;
+constexpr unsigned kSpinLimit = 4000000;  // polls of about 0.7 us each: some seconds
+constexpr size_t kMaxSmem = 227 * 1024;
+constexpr size_t kStaticSmem = 3072;  // static shared variables of the kernel, rounded up
+// Shared memory and L1 share an SM's 256 KB: larger windows slow the particle
+// loads, so that larger batches run as several groups of instances, one launch
+// after the other, whose equal shares of the rows stay within this size.  The
+// windows may take up to 8/5 of it where bands of equal cost differ in rows.
+// Measured on 48 instances of 40K to 120K particles on 128^2 beside 16 of 128K
+// on 128x256 (us per substep; shares of 200, 109, 80 and 65 KB): 1 group 325,
+// 2: 293, 3: 273, 4: 287; at 5/4 of the share 302 and 282 for 2 and 3 (some
+// re-sorts fell back to spans of equal windows).
+constexpr size_t kSoftSmem = 96 * 1024;
+
+struct SpanGroup {
+  int32_t m0, m1;    // instances
+  int32_t row0, rows;  // rows of those instances in the concatenation of all
+  int32_t n_cta;
+  int32_t pad;
+};
+
+}  // namespace
+
+// Device and host state of the span path of one engine.
+struct JfSpan {
+  std::vector<SpanGroup> groups;
+  int32_t threads = 0;     // threads of a CTA
+  int32_t n_cta = 0;       // CTAs of a launch (table stride)
+  int32_t nx_max = 0;
+  int32_t total_rows = 0;
+  int32_t cap_nodes = 0;   // window nodes of a CTA
+  size_t smem = 0;
+  SpanGroup* d_groups = nullptr;
+  int32_t* d_rowoff = nullptr;    // M + 1: first row of each instance
+  int32_t* d_rowcost = nullptr;   // total_rows
+  unsigned long long* d_rowpre = nullptr;  // total_rows: inclusive prefix of the costs within a group
+  int32_t* d_ovrow = nullptr;     // total_rows + M: overflow list starts per row (ny + 1 per instance)
+  int32_t* d_ovcur = nullptr;     // total_rows: cursors of the rows' overflow lists
+  int32_t* d_fallback = nullptr;  // groups x (n_cta + 1): cuts by window size alone
+  int4* d_seg = nullptr;          // groups x n_cta x kMaxSeg: (instance, first row, end row, 0)
+  int32_t* d_nseg = nullptr;      // groups x n_cta
+  int32_t* d_nbar = nullptr;      // M: CTAs that hold a band of the instance
+  uint32_t* d_bar = nullptr;      // 2 M: arrivals at the substep's meeting, at the drift meeting
+  int32_t* d_drift = nullptr;     // 3 M: drift flag of a substep (mod 3)
+  int32_t* d_abort = nullptr;
+  float4* d_spill = nullptr;      // 3 x total nodes
+  float4* d_slot = nullptr;       // n_cta x 2 sides x 2 parities x kOverlap x nx_max
+};
+
+namespace {
+
+struct SpanArgs {
+  JfInst I;                   // the constants that follow from n_grid, dt and the flags: the same for every instance
+  const JfInst* inst;
+  const JfParams* params;
+  JfMaterials mats;
+  float4* xv;
+  float4* C;
+  float4* F;
+  const int32_t* mat;
+  float* Jp;
+  const float2* fiber;
+  float* glow;
+  const float* rref;
+  const int32_t* cell_start;  // M x stride: start of each bin's run (relative to p_off)
+  const int32_t* cap;
+  const int32_t* ovlist;      // overflow positions (relative to p_off), grouped by row
+  const int32_t* ovrow;
+  const int32_t* rowoff;
+  const int4* seg;            // of this group
+  const int32_t* nseg;
+  const int32_t* nbar;
+  uint32_t* bar;
+  int32_t* drift;
+  int32_t* abort;
+  float4* spill;
+  float4* slot;
+  float4* grid;               // grid of the chunk's last substep, node = g_off + j * nx + i
+  int32_t* err;
+  unsigned long long* path;
+  const float* t_dev;
+  int64_t nodes;              // nodes of all instances (stride of the spill grids)
+  int32_t M;
+  int32_t nx_max;
+  int32_t stride;
+  int32_t K;
+  float dt;
+};
+
+// A band as its CTA holds it.
+struct SpanSeg {
+  JfInst I;
+  JfParams P;
+  int m, lo, hi;
+  int off;               // first node of its window in the CTA's planes
+  int segs;              // 32-cell segments of a row
+  int cap;
+  int n_bar;             // CTAs of the instance
+  int n_meet2;           // drift meetings so far
+  int ov_beg, n_ov;      // its part of the overflow list
+  int oor_beg, n_oor;    // live particles outside every stencil range (the instance's last band takes them)
+  int gen0, n_gen;       // generic tasks: first, count
+  int cell0;             // first cell task
+  __device__ __forceinline__ bool lower() const { return lo > 0; }
+  __device__ __forceinline__ bool upper() const { return hi < I.ny; }
+  // window rows that the band updates by itself: the others overlap a neighbour
+  __device__ __forceinline__ int in_lo() const { return lower() ? kOverlap : kHaloLo; }
+  __device__ __forceinline__ int in_hi() const { return hi - lo + (upper() ? 0 : kHaloLo); }
+};
+
+// The window of a band; rows outside it are reached through the published
+// grid and the spill grid.
+struct SpanWindow : JfWindow {
+  const SpanArgs& a;
+  const SpanSeg& S;
+  const int& s;  // the substep
+  __device__ __forceinline__ float2 far_gather(int i, int j) const {
+    const float4 g = __ldcg(a.grid + S.I.g_off + (int64_t)j * S.I.nx + i);
+    return make_float2(g.x, g.y);
+  }
+  __device__ __forceinline__ void far_scatter(int i, int j, float3 c, float h, bool) const {
+    const int r = s % 3;
+    atomicAdd(a.spill + r * a.nodes + S.I.g_off + (int64_t)j * S.I.nx + i, make_float4(c.x, c.y, c.z, h));
+    *(volatile int32_t*)(a.drift + 3 * S.m + r) = 1;
+  }
+};
+
+__device__ __forceinline__ void arrive(uint32_t* p) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+}
+
+// Waits until *p has reached `target` (counters only grow within a launch);
+// false when the wait gave up or another CTA did.
+__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t target, int32_t* abort) {
+  for (unsigned n = 0; n < kSpinLimit; ++n) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    if ((int32_t)(v - target) >= 0) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      return true;
+    }
+    if ((n & 63u) == 63u && *(volatile int32_t*)abort != 0) return false;
+  }
+  atomicExch(abort, 1);
+  return false;
+}
+
+// kTmem: the node blocks live in TMEM (544 .. 768 threads); otherwise in
+// registers (up to 512 threads, the default).  What bounds the pass is the
+// latency and the issue rate of the particles' FP32 chains at 16 warps per SM,
+// not memory: the state of the batch lives in L2.  Measured (us per substep,
+// 80K-slot tanks on 128^2, one cluster per instance before): 32 instances 98 ->
+// 82, 16: 107 -> 46, 8: 63 -> 27, 1: 35 -> 21.
+template <bool kTmem, bool kAxisym, bool kGlow>
+__global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(const __grid_constant__ SpanArgs a) {
+  extern __shared__ float4 smem4[];
+  __shared__ SpanSeg s_seg[kMaxSeg];
+  __shared__ float s_pressure[2][kMaxSeg];  // double-buffered: substep s + 1's are set while s is finished
+  __shared__ int s_next_task[2];
+  __shared__ int s_drift[2][kMaxSeg];
+  __shared__ int s_tot[4];                  // generic tasks, all tasks, window nodes, a wait gave up
+  __shared__ unsigned s_path[4];
+  __shared__ uint32_t s_tmem;
+
+  const int cta = blockIdx.x;
+  const int nseg = a.nseg[cta];
+  if (nseg == 0) return;
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const int lane = tid & 31, warp = tid >> 5, n_warps = nth >> 5;
+  if (tid < nseg) {
+    SpanSeg& S = s_seg[tid];
+    const int4 q = a.seg[cta * kMaxSeg + tid];
+    S.m = q.x;
+    S.lo = q.y;
+    S.hi = q.z;
+    S.I = a.inst[q.x];
+    S.P = a.params[q.x];
+    S.segs = (S.I.nx + 31) >> 5;
+    S.cap = a.cap[q.x];
+    S.n_bar = a.nbar[q.x];
+    S.n_meet2 = 0;
+    const int32_t* ovr = a.ovrow + a.rowoff[q.x] + q.x;
+    S.ov_beg = ovr[q.y];
+    S.n_ov = ovr[q.z] - S.ov_beg;
+    S.oor_beg = 0;
+    S.n_oor = 0;
+    if (q.z == S.I.ny) {
+      const int32_t* cs = a.cell_start + (int64_t)q.x * a.stride + S.I.nx * S.I.ny;
+      S.oor_beg = cs[0];
+      S.n_oor = cs[1] - cs[0];
+    }
+    S.n_gen = (S.n_ov + S.n_oor + 31) >> 5;
+    s_drift[0][tid] = s_drift[1][tid] = 0;
+  }
+  if (tid < 4) s_path[tid] = 0u;
+  __syncthreads();
+  float t = *a.t_dev;
+  if (tid == 0) {
+    int gen = 0, cell = 0, off = 0;
+    for (int q = 0; q < nseg; ++q) {
+      SpanSeg& S = s_seg[q];
+      S.gen0 = gen;
+      S.cell0 = cell;
+      S.off = off;
+      gen += S.n_gen;
+      cell += (S.hi - S.lo) * S.segs;
+      off += (S.hi - S.lo + kHalo) * S.I.nx;
+    }
+    s_tot[0] = gen;
+    s_tot[1] = gen + cell;
+    s_tot[2] = off;
+    s_tot[3] = 0;
+    s_next_task[0] = n_warps;
+  }
+  if (tid < nseg)
+    s_pressure[0][tid] = s_seg[tid].P.actuation * jf_activation(s_seg[tid].P.freq, s_seg[tid].P.contraction, t);
+  uint32_t tm_cols = 32, tm_base = 0, ta = 0;
+  if constexpr (kTmem) {
+    // one CTA per SM (its registers fill it), so the allocation never waits for another CTA's
+    const int per_quad = (n_warps + 3) >> 2;
+    while (tm_cols < (uint32_t)(48 * per_quad)) tm_cols <<= 1;
+    if (warp == 0) tm_alloc(&s_tmem, tm_cols);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  __syncthreads();
+  if constexpr (kTmem) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tm_base = s_tmem;
+    ta = tm_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(48 * (warp >> 2));
+  }
+  const int n_gen = s_tot[0], n_tasks = s_tot[1], WN = s_tot[2];
+  float2* const G = reinterpret_cast<float2*>(smem4);
+  float* const Ax = reinterpret_cast<float*>(smem4) + 2 * WN;
+  float* const Ay = Ax + WN;
+  float* const Am = Ay + WN;
+  float* const Ah = Am + WN;  // a sixth plane exists only in the axisymmetric variant
+  for (int n = tid; n < (kAxisym ? 6 : 5) * WN; n += nth) reinterpret_cast<float*>(smem4)[n] = 0.0f;
+  __syncthreads();
+
+  const int64_t slot_n = (int64_t)kOverlap * a.nx_max;
+
+  for (int s = 0; s <= a.K; ++s) {
+    const bool do_g2p = s > 0;
+    const bool do_p2g = s < a.K;
+
+    // a warp claims tasks from a shared counter: groups of 32 generic particles
+    // first, lanes far apart in the list, then the 32-cell row segments
+    for (int task = warp; task < n_tasks;) {
+      const bool generic = task < n_gen;
+      int q = 0;
+      if (generic) {
+        while (q + 1 < nseg && task >= s_seg[q + 1].gen0) ++q;
+      } else {
+        while (q + 1 < nseg && task - n_gen >= s_seg[q + 1].cell0) ++q;
+      }
+      const SpanSeg& S = s_seg[q];
+      // kernel parameters where the instances agree: operands of the arithmetic that take no registers
+      JfInst I = a.I;
+      I.axisym = kAxisym;
+      I.ny = S.I.ny;
+      I.y_hi = S.I.y_hi;
+      const JfEnv<SpanArgs> E{I, a, S.P.payload_density, kGlow};
+      const SpanWindow w{{G + S.off, Ax + S.off, Ay + S.off, Am + S.off, Ah + S.off, I.nx, S.lo - kHaloLo,
+                          S.hi - S.lo + kHalo},
+                         a, S, s};
+      const float pressure = s_pressure[s & 1][q];
+      bool nonfinite = false;
+      // the lane's particles, as engine positions
+      int beg = 0, end = 0, cy = 0, seg0 = 0;
+      const int p0 = (int)S.I.p_off;
+      if (generic) {
+        const int e = task - S.gen0 + lane * S.n_gen;
+        if (e < S.n_ov + S.n_oor) {
+          const bool over = e < S.n_ov;
+          beg = p0 + (over ? a.ovlist[p0 + S.ov_beg + e] : S.oor_beg + e - S.n_ov);
+          end = beg + 1;
+          atomicAdd(&s_path[over ? 3 : 1], 1u);
+        }
+      } else {
+        const int c = task - n_gen - S.cell0;
+        const int row = c / S.segs;
+        cy = S.lo + row;
+        seg0 = (c - row * S.segs) << 5;
+        if (seg0 + lane < I.nx) {
+          const int32_t* cs = a.cell_start + (int64_t)S.m * a.stride + cy * I.nx + seg0 + lane;
+          beg = p0 + cs[0];
+          end = p0 + cs[1];
+          if (end - beg > S.cap) end = beg + S.cap;  // the rest of the cell is overflow
+        }
+      }
+      run_task<kTmem>(E, w, !generic, beg, end, cy, seg0, ta, do_g2p, do_p2g, pressure, s_path, nonfinite);
+      if (__any_sync(0xffffffffu, nonfinite) && lane == 0) atomicOr(a.err + S.m, 1);
+      int nt = 0;
+      if (lane == 0) nt = atomicAdd(&s_next_task[s & 1], 1);
+      task = __shfl_sync(0xffffffffu, nt, 0);
+    }
+    __syncthreads();
+    if (!do_p2g) break;
+    float4* const spill = a.spill + (int64_t)(s % 3) * a.nodes;
+
+    // partial sums of the rows around the cuts, for the other side
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const SpanSeg& S = s_seg[side ? nseg - 1 : 0];
+      if (!(side ? S.upper() : S.lower())) continue;
+      const int n0 = S.off + (side ? S.hi - S.lo : 0) * S.I.nx;
+      float4* const to = a.slot + ((cta * 2 + side) * 2 + (s & 1)) * slot_n;
+      for (int n = tid; n < kOverlap * S.I.nx; n += nth)
+        __stcg(to + n, make_float4(Ax[n0 + n], Ay[n0 + n], Am[n0 + n], kAxisym ? Ah[n0 + n] : 0.0f));
+    }
+    __syncthreads();
+    if (tid < nseg && s_seg[tid].n_bar > 1) arrive(a.bar + s_seg[tid].m);
+
+    // grid update of one node of band S from its sums; `own`: the band writes
+    // it to the grid in global memory where asked to
+    const bool last = (s == a.K - 1);
+    auto update_node = [&](const SpanSeg& S, int wr, int i, float mx, float my, float mm, float mh, bool publish) {
+      const int j = S.lo - kHaloLo + wr;
+      const float2 u = jf_grid_node(S.I, i, j, mx, my, mm, mh);
+      G[S.off + wr * S.I.nx + i] = u;
+      if (publish) a.grid[S.I.g_off + (int64_t)j * S.I.nx + i] = make_float4(u.x, u.y, mm, 0.0f);
+    };
+    // rows that no neighbour shares, while the counters travel.  Their sums
+    // stay until the meeting is over: a spill may come in.
+    for (int q = 0; q < nseg; ++q) {
+      const SpanSeg& S = s_seg[q];
+      const int nx = S.I.nx;
+      const int n0 = S.in_lo() * nx, n1 = S.in_hi() * nx;
+      for (int n = n0 + tid; n < n1; n += nth) {
+        const int wr = n / nx, o = S.off + n;
+        update_node(S, wr, n - wr * nx, Ax[o], Ay[o], Am[o], kAxisym ? Ah[o] : 0.0f, last);
+      }
+    }
+    if (tid < nseg) {
+      const SpanSeg& S = s_seg[tid];
+      if (S.n_bar > 1) {
+        if (!wait_for(a.bar + S.m, (uint32_t)(s + 1) * S.n_bar, a.abort)) {
+          s_tot[3] = 1;
+          atomicOr(a.err + S.m, kJfErrAbort);
+        }
+        s_drift[s & 1][tid] = *(volatile int32_t*)(a.drift + 3 * S.m + s % 3);
+      }
+    }
+    __syncthreads();
+    if (s_tot[3]) break;
+
+    // rows around the cuts: both sides' sums, and the spill
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const int q = side ? nseg - 1 : 0;
+      const SpanSeg& S = s_seg[q];
+      if (!(side ? S.upper() : S.lower())) continue;
+      const int nx = S.I.nx;
+      const int wr0 = side ? S.hi - S.lo : 0;
+      const bool drift = s_drift[s & 1][q] != 0;
+      const int other = side ? cta + 1 : cta - 1;
+      const float4* const from = a.slot + ((other * 2 + (side ^ 1)) * 2 + (s & 1)) * slot_n;
+      for (int n = tid; n < kOverlap * nx; n += nth) {
+        const int r = n / nx, i = n - r * nx;
+        const int o = S.off + wr0 * nx + n;
+        const float4 b = __ldcg(from + n);
+        float mx = Ax[o] + b.x, my = Ay[o] + b.y, mm = Am[o] + b.z, mh = kAxisym ? Ah[o] + b.w : 0.0f;
+        if (drift) {
+          const float4 e = __ldcg(spill + S.I.g_off + (int64_t)(S.lo - kHaloLo + wr0 + r) * nx + i);
+          mx += e.x;
+          my += e.y;
+          mm += e.z;
+          mh += e.w;
+        }
+        const bool own = side ? r == 0 : r > 0;
+        update_node(S, wr0 + r, i, mx, my, mm, mh, own && (last || drift));
+        Ax[o] = 0.0f;
+        Ay[o] = 0.0f;
+        Am[o] = 0.0f;
+        if (kAxisym) Ah[o] = 0.0f;
+      }
+    }
+    // the other rows: the spill where there is one, and clear sums
+    bool any_drift = false;
+    for (int q = 0; q < nseg; ++q) {
+      const SpanSeg& S = s_seg[q];
+      const int nx = S.I.nx;
+      const bool drift = s_drift[s & 1][q] != 0;
+      any_drift |= drift;
+      const int n0 = S.in_lo() * nx, n1 = S.in_hi() * nx;
+      for (int n = n0 + tid; n < n1; n += nth) {
+        const int o = S.off + n;
+        if (drift) {
+          const int wr = n / nx, i = n - wr * nx;
+          const float4 e = __ldcg(spill + S.I.g_off + (int64_t)(S.lo - kHaloLo + wr) * nx + i);
+          update_node(S, wr, i, Ax[o] + e.x, Ay[o] + e.y, Am[o] + e.z, kAxisym ? Ah[o] + e.w : 0.0f, true);
+        }
+        Ax[o] = 0.0f;
+        Ay[o] = 0.0f;
+        Am[o] = 0.0f;
+        if (kAxisym) Ah[o] = 0.0f;
+      }
+      // the spill of the substep before has been read by everyone: its rows are cleared by their owners
+      if (s > 0 && s_drift[(s - 1) & 1][q]) {
+        float4* const old = a.spill + (int64_t)((s - 1) % 3) * a.nodes + S.I.g_off + (int64_t)S.lo * nx;
+        for (int n = tid; n < (S.hi - S.lo) * nx; n += nth) __stcg(old + n, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+        if (tid == 0 && S.lo == 0) *(volatile int32_t*)(a.drift + 3 * S.m + (s - 1) % 3) = 0;
+      }
+    }
+    if (any_drift) {  // the published rows are there for everyone after a second meeting
+      __syncthreads();
+      if (tid < nseg && s_drift[s & 1][tid]) {
+        SpanSeg& S = s_seg[tid];
+        S.n_meet2 += 1;
+        arrive(a.bar + a.M + S.m);
+        if (!wait_for(a.bar + a.M + S.m, (uint32_t)S.n_meet2 * S.n_bar, a.abort)) {
+          s_tot[3] = 1;
+          atomicOr(a.err + S.m, kJfErrAbort);
+        }
+      }
+    }
+    t = t + a.dt;
+    if (tid < nseg)
+      s_pressure[(s + 1) & 1][tid] =
+          s_seg[tid].P.actuation * jf_activation(s_seg[tid].P.freq, s_seg[tid].P.contraction, t);
+    if (tid == 0) s_next_task[(s + 1) & 1] = n_warps;
+    __syncthreads();
+    if (any_drift && s_tot[3]) break;
+  }
+  // every warp is past its last access: the TMEM allocation is freed
+  if constexpr (kTmem) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if constexpr (kTmem) {
+    if (warp == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tm_free(tm_base, tm_cols);
+    }
+  }
+  if (tid < 4 && s_path[tid]) atomicAdd(a.path + tid, (unsigned long long)s_path[tid]);
+}
+
+// Per instance: the cell cap, the row costs, the overflow list's row starts,
+// the exclusive scan of the bins (counts become bin starts), and the span
+// kernel's flags and counters cleared.  One warp per 32-cell segment: its
+// counts are one coalesced load and the candidates' overflows warp sums.
+__global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
+    const JfInst* __restrict__ inst, int32_t* __restrict__ counts, int stride, const int32_t* __restrict__ solid,
+    const int32_t* __restrict__ rowoff, int32_t* __restrict__ rowcost, int32_t* __restrict__ ovrow,
+    int32_t* __restrict__ ovcur, int32_t* __restrict__ cap_out, int fixed_cap, int32_t* __restrict__ band, int CS,
+    uint32_t* __restrict__ bar, int32_t* __restrict__ drift, int32_t* __restrict__ abort, float4* __restrict__ spill,
+    int64_t nodes, int M) {
+  constexpr int kWarps = kScanThreads / 32;
+  __shared__ int s_cost[32];
+  __shared__ int s_row_cost[kJfMaxBandRows];
+  __shared__ int s_row_over[kJfMaxBandRows];
+  __shared__ int s_warp[kWarps];
+  __shared__ int s_cap;
+  const unsigned full = 0xffffffffu;
+  const int m = blockIdx.x;
+  const JfInst I = inst[m];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int32_t* c = counts + (int64_t)m * stride;
+  const int segs = (I.nx + 31) >> 5;
+  // what a chunk's last substeps may have left in the spill grids
+  for (int r = 0; r < 3; ++r)
+    if (drift[3 * m + r])
+      for (int n = tid; n < I.nx * I.ny; n += kScanThreads)
+        spill[(int64_t)r * nodes + I.g_off + n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (tid < 32) s_cost[tid] = 0;
+  for (int y = tid; y < I.ny; y += kScanThreads) {
+    s_row_cost[y] = kRowCost + (kSolidCostHalves * solid[m * kJfMaxBandRows + y]) / 2;
+    s_row_over[y] = 0;
+  }
+  __syncthreads();
+  if (tid < 3) drift[3 * m + tid] = 0;
+  if (tid < 2) bar[tid * M + m] = 0u;
+  if (tid == 0 && m == 0) *abort = 0;
+
+  // lane k sums the cost of candidate k (0 = no cap), in quarter lane-iterations
+  int cost = 0;
+  for (int sg = warp; sg < I.ny * segs; sg += kWarps) {
+    const int row = sg / segs, x = ((sg - row * segs) << 5) + lane;
+    const int n = x < I.nx ? c[row * I.nx + x] : 0;
+    const int mx = (int)__reduce_max_sync(full, (unsigned)n);
+    if (mx == 0) continue;
+    int ov = 0;
+    for (int k = 1; k < min(mx, kCapCandidates); ++k) {
+      const int o = (int)__reduce_add_sync(full, (unsigned)max(0, n - k));
+      if (lane == k) ov = o;
+    }
+    cost += 128 * (lane == 0 ? mx : min(mx, lane)) + 6 * ov;
+  }
+  if (lane < kCapCandidates) atomicAdd(&s_cost[lane], cost);
+  __syncthreads();
+  if (tid == 0) {
+    int best = 0;
+    for (int k = 1; k < kCapCandidates; ++k)
+      if (s_cost[k] < s_cost[best]) best = k;
+    if (fixed_cap > 0) best = fixed_cap < kCapCandidates ? fixed_cap : 0;
+    s_cap = best == 0 ? kNoCap : best;
+    cap_out[m] = s_cap;
+  }
+  __syncthreads();
+  const int cap = s_cap;
+  for (int sg = warp; sg < I.ny * segs; sg += kWarps) {
+    const int row = sg / segs, x = ((sg - row * segs) << 5) + lane;
+    const int n = x < I.nx ? c[row * I.nx + x] : 0;
+    const int mx = (int)__reduce_max_sync(full, (unsigned)n);
+    const int ov = (int)__reduce_add_sync(full, (unsigned)max(0, n - cap));
+    if (lane == 0 && mx) {
+      atomicAdd(&s_row_cost[row], 128 * min(mx, cap) + 6 * ov);
+      if (ov) atomicAdd(&s_row_over[row], ov);
+    }
+  }
+  __syncthreads();
+
+  // block scan of one value per thread
+  auto block_exclusive = [&](int v) {
+    int incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(full, incl, off);
+      if (lane >= off) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      int w = s_warp[lane];
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(full, w, off);
+        if (lane >= off) w += y;
+      }
+      s_warp[lane] = w;
+    }
+    __syncthreads();
+    const int r = incl - v + (warp > 0 ? s_warp[warp - 1] : 0);
+    __syncthreads();
+    return r;
+  };
+  static_assert(kJfMaxBandRows <= kScanThreads, "one row per thread");
+  {
+    const int over = tid < I.ny ? s_row_over[tid] : 0;
+    const int start = block_exclusive(over);
+    if (tid < I.ny) {
+      const int r = rowoff[m] + tid;
+      rowcost[r] = s_row_cost[tid];
+      ovrow[r + m] = start;
+      ovcur[r] = start;
+      if (tid == I.ny - 1) ovrow[r + m + 1] = start + over;
+    }
+  }
+  // bins: each warp takes a run of 32-bin tiles
+  const int nbins = I.nx * I.ny + 2;
+  const int tiles = (nbins + 31) >> 5, per = (tiles + kWarps - 1) / kWarps;
+  const int t0 = min(warp * per, tiles), t1 = min(t0 + per, tiles);
+  int sum = 0;
+  for (int q = t0; q < t1; ++q) {
+    const int b = (q << 5) + lane;
+    sum += b < nbins ? c[b] : 0;
+  }
+  sum = (int)__reduce_add_sync(full, (unsigned)sum);
+  const int before = block_exclusive(lane == 0 ? sum : 0);
+  int run = __shfl_sync(full, before, 0);
+  for (int q = t0; q < t1; ++q) {
+    const int b = (q << 5) + lane;
+    const int n = b < nbins ? c[b] : 0;
+    int incl = n;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(full, incl, off);
+      if (lane >= off) incl += y;
+    }
+    if (b < nbins) c[b] = run + incl - n;
+    if (b == nbins - 1) band[m * (CS + 1) + CS] = (int32_t)I.p_off + run + incl - n;  // first dead slot
+    run += __shfl_sync(full, incl, 31);
+  }
+}
+
+// One block per group: the costs' prefix over the group's rows, cut into spans
+// of equal cost, each cut moved so that every band has at least kMinRows rows
+// and every CTA's windows fit (where that cannot be had, the cuts by window
+// size alone), and the CTAs' band table.
+__global__ void __launch_bounds__(kScanThreads) span_cut_kernel(
+    const SpanGroup* __restrict__ groups, const JfInst* __restrict__ inst, const int32_t* __restrict__ rowoff,
+    const int32_t* __restrict__ rowcost, unsigned long long* __restrict__ rowpre, int cap_nodes, int n_cta_max,
+    const int32_t* __restrict__ fallback, int4* __restrict__ seg, int32_t* __restrict__ nseg,
+    int32_t* __restrict__ nbar) {
+  __shared__ unsigned long long s_sum[kScanThreads / 32];
+  __shared__ int s_cut[kScanThreads + 1];
+  __shared__ int s_used;
+  const SpanGroup g = groups[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned full = 0xffffffffu;
+  const int32_t* cost = rowcost + g.row0;
+  unsigned long long* pre = rowpre + g.row0;
+  const int per = (g.rows + kScanThreads - 1) / kScanThreads;
+  const int r0 = min(tid * per, g.rows), r1 = min(r0 + per, g.rows);
+  unsigned long long sum = 0;
+  for (int r = r0; r < r1; ++r) sum += (unsigned)cost[r];
+  unsigned long long incl = sum;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned long long y = __shfl_up_sync(full, incl, off);
+    if (lane >= off) incl += y;
+  }
+  if (lane == 31) s_sum[warp] = incl;
+  for (int m = g.m0 + tid; m < g.m1; m += kScanThreads) nbar[m] = 0;
+  __syncthreads();
+  unsigned long long run = incl - sum, total = 0;
+  for (int w = 0; w < kScanThreads / 32; ++w) {
+    if (w < warp) run += s_sum[w];
+    total += s_sum[w];
+  }
+  for (int r = r0; r < r1; ++r) {
+    run += (unsigned)cost[r];
+    pre[r] = run;
+  }
+  __syncthreads();
+  // span c starts where the cost before it reaches c / n_cta of the total
+  if (tid > 0 && tid < g.n_cta) {
+    const unsigned long long target = total * (unsigned)tid / (unsigned)g.n_cta;
+    int lo = 0, hi = g.rows;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (pre[mid] - (unsigned)cost[mid] / 2 < target) lo = mid + 1;
+      else hi = mid;
+    }
+    s_cut[tid] = lo;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int prev = 0, used = 0, m = g.m0;
+    bool ok = true;
+    for (int q = 1; q <= g.n_cta && prev < g.rows; ++q) {
+      int y = q < g.n_cta ? s_cut[q] : g.rows;
+      // instance of the span's first row, its rows [b, e) in the group
+      int b = rowoff[m] - g.row0, e = rowoff[m + 1] - g.row0;
+      while (prev >= e) {
+        ++m;
+        b = e;
+        e = rowoff[m + 1] - g.row0;
+      }
+      if (y < prev + kMinRows) y = prev + kMinRows;
+      // walk its bands while they fit
+      int at = prev, mm = m, bb = b, ee = e, room = cap_nodes, left = kMaxSeg;
+      for (;;) {
+        const int nx = inst[mm].nx;
+        int stop = min(y, ee);
+        // a cut leaves at least kMinRows rows on either side within an instance
+        if (stop < ee && ee - stop < kMinRows) stop = ee;
+        if (stop < ee && stop - bb < kMinRows) stop = at > prev ? at : bb + kMinRows;
+        if (left == 0) stop = at;
+        if (stop > at && (stop - at + kHalo) * nx > room) {
+          stop = at + room / nx - kHalo;
+          if (ee - stop < kMinRows) stop = ee - kMinRows;
+          if (stop - at < kMinRows) stop = at;
+        }
+        if (stop > at) {
+          room -= (stop - at + kHalo) * nx;
+          --left;
+        }
+        at = stop;
+        if (at < ee || at >= y || at >= g.rows) break;
+        ++mm;
+        bb = ee;
+        ee = rowoff[mm + 1] - g.row0;
+      }
+      if (at <= prev) {
+        ok = false;
+        break;
+      }
+      s_cut[used++] = prev;  // span `used`: s_cut[used] is read above only for larger q
+      prev = at;
+    }
+    if (prev < g.rows) ok = false;
+    s_used = ok ? used : -1;
+    if (ok) s_cut[used] = g.rows;
+  }
+  __syncthreads();
+  const int used = s_used;
+  const int32_t* fb = fallback + blockIdx.x * (n_cta_max + 1);
+  for (int q = tid; q < n_cta_max; q += kScanThreads) {
+    const int lo = used >= 0 ? (q < used ? s_cut[q] : g.rows) : fb[q];
+    const int hi = used >= 0 ? (q < used ? s_cut[q + 1] : g.rows) : fb[q + 1];
+    int n = 0;
+    if (lo < hi) {
+      int m = g.m0, top = g.m1;  // instance of row lo
+      while (top - m > 1) {
+        const int mid = (m + top) >> 1;
+        if (rowoff[mid] - g.row0 <= lo) m = mid;
+        else top = mid;
+      }
+      for (int at = lo; at < hi; ++m) {
+        const int b = rowoff[m] - g.row0, e = rowoff[m + 1] - g.row0;
+        const int stop = min(hi, e);
+        seg[((int64_t)blockIdx.x * n_cta_max + q) * kMaxSeg + n] = make_int4(m, at - b, stop - b, 0);
+        atomicAdd(nbar + m, 1);
+        ++n;
+        at = stop;
+      }
+    }
+    nseg[blockIdx.x * n_cta_max + q] = n;
+  }
+}
+
+// Moves every particle to bin start + rank; particles of a cell beyond the
+// cap are also listed in their row's part of the overflow list.
+__global__ void __launch_bounds__(kMoveThreads) span_move_kernel(
+    const JfInst* __restrict__ inst, const int32_t* __restrict__ keys, const int32_t* __restrict__ rank,
+    const int32_t* __restrict__ starts, int stride, const int32_t* __restrict__ cap,
+    const int32_t* __restrict__ rowoff, int32_t* __restrict__ ovcur, int32_t* __restrict__ ovlist, JfParticles src,
+    JfParticles dst) {
+  const int m = blockIdx.y;
+  const JfInst I = inst[m];
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= I.n_slots) return;
+  const int64_t g = I.p_off + k;
+  const int key = keys[g];
+  const int rk = rank[g];
+  const int32_t rel = starts[(int64_t)m * stride + key] + rk;
+  const int64_t d = I.p_off + rel;
+  if (key < I.nx * I.ny && rk >= cap[m])
+    ovlist[I.p_off + atomicAdd(ovcur + rowoff[m] + key / I.nx, 1)] = rel;
+  dst.xv[d] = src.xv[g];
+  dst.C[d] = src.C[g];
+  dst.F[d] = src.F[g];
+  dst.mat[d] = src.mat[g];
+  dst.fiber[d] = src.fiber[g];
+  dst.Jp[d] = src.Jp[g];
+  dst.glow[d] = src.glow[g];
+  dst.slot[d] = src.slot[g];
+  dst.rref[d] = src.rref[g];
+}
+
+using SpanKernel = void (*)(const SpanArgs);
+
+// the instantiation for the launch's CTA size and the engine's flags
+SpanKernel span_kernel_for(const jf_engine* e, int threads) {
+  const bool axisym = e->flags & JF_FLAG_AXISYM, glow = e->flags & JF_FLAG_GLOW;
+  if (threads > 512)
+    return axisym ? (glow ? span_kernel<true, true, true> : span_kernel<true, true, false>)
+                  : (glow ? span_kernel<true, false, true> : span_kernel<true, false, false>);
+  return axisym ? (glow ? span_kernel<false, true, true> : span_kernel<false, true, false>)
+                : (glow ? span_kernel<false, false, true> : span_kernel<false, false, false>);
+}
+
+// Spans of the group by window size alone; false when n_cta spans do not do.
+bool fill_cuts(const jf_engine* e, const SpanGroup& g, const std::vector<int32_t>& rowoff, int cap_nodes,
+               std::vector<int32_t>& cuts) {
+  cuts.assign(1, 0);
+  int room = cap_nodes, left = kMaxSeg;
+  for (int m = g.m0; m < g.m1; ++m) {
+    const int nx = e->inst[m].nx, ny = e->inst[m].ny, b = rowoff[m] - g.row0;
+    int y = 0;
+    while (y < ny) {
+      int rows = left > 0 ? std::min(room / nx - kHalo, ny - y) : 0;
+      if (ny - y - rows > 0 && ny - y - rows < kMinRows) rows = ny - y - kMinRows;
+      if (rows < kMinRows) {
+        if (cuts.back() == b + y) return false;  // an empty span: a band does not fit
+        cuts.push_back(b + y);
+        room = cap_nodes;
+        left = kMaxSeg;
+        continue;
+      }
+      room -= (rows + kHalo) * nx;
+      --left;
+      y += rows;
+    }
+  }
+  if ((int)cuts.size() > g.n_cta) return false;
+  cuts.resize(g.n_cta + 1, g.rows);
+  return true;
+}
+
+template <class T>
+cudaError_t dev(T** p, size_t n) {
+  return cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(n, 1));
+}
+
+}  // namespace
+
+void jf_span_free(jf_engine* e) {
+  JfSpan* s = e->span;
+  if (!s) return;
+  cudaFree(s->d_groups); cudaFree(s->d_rowoff); cudaFree(s->d_rowcost); cudaFree(s->d_rowpre); cudaFree(s->d_ovrow);
+  cudaFree(s->d_ovcur); cudaFree(s->d_fallback); cudaFree(s->d_seg); cudaFree(s->d_nseg); cudaFree(s->d_nbar);
+  cudaFree(s->d_bar); cudaFree(s->d_drift); cudaFree(s->d_abort); cudaFree(s->d_spill); cudaFree(s->d_slot);
+  delete s;
+  e->span = nullptr;
+}
+
+// Sets the span path up (e->span), or leaves it off where the batch does not
+// suit it: grids taller than the row tables, instances of different n_grid
+// (the kernel's constants are launch parameters), rows too wide for a band of
+// 4 rows and its halo, or a device without cooperative launches.
+cudaError_t jf_span_setup(jf_engine* e, int threads) {
+  if (threads == 0) threads = kSpanThreads;
+  int n_sm = 0, coop = 0;
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, e->device);
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->device);
+  if (!coop || n_sm < 1) return cudaSuccess;
+  n_sm = std::min(n_sm, kScanThreads);
+  std::vector<int32_t> rowoff(1, 0);
+  int nx_max = 0;
+  for (const JfInst& I : e->inst) {
+    if (I.ny > kJfMaxBandRows || I.nx != e->inst[0].nx) return cudaSuccess;
+    if (rowoff.back() > (1 << 28)) return cudaSuccess;
+    rowoff.push_back(rowoff.back() + I.ny);
+    nx_max = std::max(nx_max, I.nx);
+  }
+  const size_t node_bytes = sizeof(float) * ((e->flags & JF_FLAG_AXISYM) ? 6 : 5);
+  const int64_t hard = (int64_t)((kMaxSmem - kStaticSmem) / node_bytes);
+  const int64_t soft = std::min<int64_t>(hard, (int64_t)(kSoftSmem / node_bytes));
+
+  // as few groups of consecutive instances as keep a CTA's share of the rows
+  // within the soft size
+  std::vector<SpanGroup> groups;
+  int64_t need = 0;
+  for (int n_groups = 1; n_groups <= e->M; n_groups = n_groups < 8 ? n_groups + 1 : n_groups * 2) {
+    groups.clear();
+    need = 0;
+    int m = 0;
+    for (int k = 0; k < n_groups && m < e->M; ++k) {
+      SpanGroup g = {};
+      g.m0 = m;
+      const int64_t upto = rowoff[e->M] * (int64_t)(k + 1) / n_groups;
+      do ++m;
+      while (m < e->M && (k == n_groups - 1 || rowoff[m + 1] <= upto));
+      g.m1 = m;
+      g.row0 = rowoff[g.m0];
+      g.rows = rowoff[m] - g.row0;
+      g.n_cta = std::max(1, std::min(n_sm, g.rows / kMinRows));
+      int64_t nodes = 0;
+      for (int q = g.m0; q < g.m1; ++q) nodes += (int64_t)e->inst[q].nx * e->inst[q].ny;
+      // a CTA's share and its halo, twice where its span holds the end of one instance and the start of the next
+      const int64_t share = nodes / g.n_cta + (g.m1 - g.m0 > 1 ? 2 : 1) * kHalo * nx_max;
+      need = std::max(need, share);
+      groups.push_back(g);
+    }
+    if (need <= soft) break;
+  }
+  int64_t cap = std::max<int64_t>(need + need * 3 / 5, (int64_t)(4 * kMinRows + kHalo) * nx_max);
+  cap = std::min(cap, hard);
+  std::vector<int32_t> table, cuts;
+  int n_cta = 0;
+  for (const SpanGroup& g : groups) n_cta = std::max(n_cta, g.n_cta);
+  for (const SpanGroup& g : groups) {
+    if (!fill_cuts(e, g, rowoff, (int)cap, cuts)) {
+      cap = hard;
+      if (!fill_cuts(e, g, rowoff, (int)cap, cuts)) return cudaSuccess;
+    }
+    cuts.resize(n_cta + 1, g.rows);
+    table.insert(table.end(), cuts.begin(), cuts.end());
+  }
+  const size_t smem = node_bytes * (size_t)cap;
+  const void* k = (const void*)span_kernel_for(e, threads);
+  cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int blocks = 0;
+  if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, threads, smem);
+  if (err != cudaSuccess) return err;
+  if (blocks < 1) return cudaSuccess;
+
+  JfSpan* s = new JfSpan();
+  e->span = s;
+  s->threads = threads;
+  s->groups = groups;
+  s->n_cta = n_cta;
+  s->nx_max = nx_max;
+  s->total_rows = rowoff[e->M];
+  s->cap_nodes = (int32_t)cap;
+  s->smem = smem;
+  const size_t ng = groups.size(), rows = (size_t)s->total_rows, M = (size_t)e->M;
+  if ((err = dev(&s->d_groups, ng)) || (err = dev(&s->d_rowoff, M + 1)) || (err = dev(&s->d_rowcost, rows)) ||
+      (err = dev(&s->d_rowpre, rows)) || (err = dev(&s->d_ovrow, rows + M)) || (err = dev(&s->d_ovcur, rows)) ||
+      (err = dev(&s->d_fallback, table.size())) || (err = dev(&s->d_seg, ng * n_cta * kMaxSeg)) ||
+      (err = dev(&s->d_nseg, ng * n_cta)) || (err = dev(&s->d_nbar, M)) || (err = dev(&s->d_bar, 2 * M)) ||
+      (err = dev(&s->d_drift, 3 * M)) || (err = dev(&s->d_abort, 1)) ||
+      (err = dev(&s->d_spill, 3 * (size_t)e->total_nodes)) ||
+      (err = dev(&s->d_slot, (size_t)n_cta * 4 * kOverlap * nx_max)))
+    return err;
+  if ((err = cudaMemcpy(s->d_groups, groups.data(), sizeof(SpanGroup) * ng, cudaMemcpyHostToDevice)) ||
+      (err = cudaMemcpy(s->d_rowoff, rowoff.data(), sizeof(int32_t) * (M + 1), cudaMemcpyHostToDevice)) ||
+      (err = cudaMemcpy(s->d_fallback, table.data(), sizeof(int32_t) * table.size(), cudaMemcpyHostToDevice)) ||
+      (err = cudaMemset(s->d_drift, 0, sizeof(int32_t) * 3 * M)) ||
+      (err = cudaMemset(s->d_spill, 0, sizeof(float4) * 3 * (size_t)std::max<int64_t>(e->total_nodes, 1))))
+    return err;
+  return cudaSuccess;
+}
+
+// The part of a re-sort after the cell keys: bins, spans, and the particles
+// moved into the other buffer set.
+cudaError_t jf_span_sort(jf_engine* e) {
+  JfSpan* s = e->span;
+  const int stride = e->max_cells + 2;
+  span_scan_kernel<<<e->M, kScanThreads, 0, e->stream>>>(
+      e->d_inst, e->d_counts, stride, e->d_solid, s->d_rowoff, s->d_rowcost, s->d_ovrow, s->d_ovcur, e->d_cap,
+      e->cell_cap, e->d_band, e->cluster, s->d_bar, s->d_drift, s->d_abort, s->d_spill, e->total_nodes, e->M);
+  span_cut_kernel<<<(int)s->groups.size(), kScanThreads, 0, e->stream>>>(
+      s->d_groups, e->d_inst, s->d_rowoff, s->d_rowcost, s->d_rowpre, s->cap_nodes, s->n_cta, s->d_fallback, s->d_seg,
+      s->d_nseg, s->d_nbar);
+  if (e->max_slots > 0) {
+    const dim3 grid((e->max_slots + kMoveThreads - 1) / kMoveThreads, e->M);
+    span_move_kernel<<<grid, kMoveThreads, 0, e->stream>>>(e->d_inst, e->d_keys, e->d_rank, e->d_counts, stride,
+                                                          e->d_cap, s->d_rowoff, s->d_ovcur, e->d_ovlist, e->p, e->q);
+  }
+  return cudaGetLastError();
+}
+
+// K substeps of every instance: one cooperative launch per group.
+cudaError_t jf_span_launch(jf_engine* e, int K) {
+  JfSpan* s = e->span;
+  SpanArgs a;
+  a.I = e->inst[0];
+  a.inst = e->d_inst;
+  a.params = e->d_params;
+  a.mats = jf_materials();
+  a.xv = e->p.xv;
+  a.C = e->p.C;
+  a.F = e->p.F;
+  a.mat = e->p.mat;
+  a.Jp = e->p.Jp;
+  a.fiber = e->p.fiber;
+  a.glow = e->p.glow;
+  a.rref = e->p.rref;
+  a.cell_start = e->d_counts;
+  a.cap = e->d_cap;
+  a.ovlist = e->d_ovlist;
+  a.ovrow = s->d_ovrow;
+  a.rowoff = s->d_rowoff;
+  a.nbar = s->d_nbar;
+  a.bar = s->d_bar;
+  a.drift = s->d_drift;
+  a.abort = s->d_abort;
+  a.spill = s->d_spill;
+  a.slot = s->d_slot;
+  a.grid = e->d_grid;
+  a.err = e->d_err;
+  a.path = e->d_path;
+  a.t_dev = e->d_time;
+  a.nodes = e->total_nodes;
+  a.M = e->M;
+  a.nx_max = s->nx_max;
+  a.stride = e->max_cells + 2;
+  a.K = K;
+  a.dt = (float)e->dt;
+  for (size_t g = 0; g < s->groups.size(); ++g) {
+    a.seg = s->d_seg + g * s->n_cta * kMaxSeg;
+    a.nseg = s->d_nseg + g * s->n_cta;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s->groups[g].n_cta, 1, 1);
+    cfg.blockDim = dim3(s->threads, 1, 1);
+    cfg.dynamicSmemBytes = s->smem;
+    cfg.stream = e->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, span_kernel_for(e, s->threads), a);
+    if (err != cudaSuccess) return err;
+    e->launches += 1;
+  }
+  return cudaSuccess;
+}

@@ -51,8 +51,9 @@ def _choice(table, value, what):
 class Engine:
     """A batch of independent MLS-MPM instances on one GPU.
 
-    ``path='batched'`` advances every instance in one persistent cluster launch
-    per chunk; ``path='plain'`` launches clear / P2G / grid update / G2P per
+    ``path='batched'`` advances every instance in one persistent launch per
+    chunk (the batch's grid rows cut into one span per SM, or, with a
+    ``cluster_size``, one thread-block cluster per instance); ``path='plain'`` launches clear / P2G / grid update / G2P per
     instance and substep, as the reference's substep() offloads do.
     ``axisym=True`` runs the axisymmetric (r, z) substep of JELLY_AXISYM=1
     (every instance; the load positions' x becomes each particle's r_ref).
@@ -143,8 +144,10 @@ class Engine:
                 "remote_gathers": int(out[2]), "overflow_scatters": int(out[3])}
 
     def layout(self) -> dict:
-        """The batched launch layout the engine chose: CTAs per instance and
-        threads per CTA (above 512 the cell lanes' node blocks live in TMEM)."""
+        """The cluster layout of the batch: CTAs per instance and threads per CTA
+        (above 512 the cell lanes' node blocks live in TMEM).  Without a
+        cluster_size the batch runs as spans where it can, which use 512
+        threads unless block_threads was given."""
         cs, bt = np.zeros(1, np.int32), np.zeros(1, np.int32)
         self._check(self._lib.jf_get_layout(self._h, _ptr(cs), _ptr(bt)))
         return {"cluster_size": int(cs[0]), "block_threads": int(bt[0])}
