@@ -738,9 +738,10 @@ static const void* chunk_kernel_for(const jf_engine* e) {
 }
 
 cudaError_t jf_batched_prepare(jf_engine* e) {
-  const size_t smem = jf_batched_smem_bytes(e);
   const void* k = chunk_kernel_for(e);
-  cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the attribute belongs to the kernel, not to the engine: the most any
+  // engine may take (227 KB less the static variables, as jf_create checks)
+  cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
   if (err != cudaSuccess) return err;
   if (e->cluster > 8) {
     err = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

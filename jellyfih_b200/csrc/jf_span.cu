@@ -907,7 +907,9 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
   }
   const size_t smem = node_bytes * (size_t)cap;
   const void* k = (const void*)span_kernel_for(e, threads);
-  cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the attribute belongs to the kernel, not to the engine: the most any engine may take
+  cudaError_t err =
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMaxSmem - kStaticSmem));
   int blocks = 0;
   if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, threads, smem);
   if (err != cudaSuccess) return err;

@@ -85,3 +85,16 @@ def test_spans_carry_a_chunk_as_clusters_do():
         rows.append(e.run_headless(48))
         e.close()
     assert np.abs(rows[0] - rows[1]).max() <= 1e-6
+
+
+@pytest.mark.parametrize("cluster_size", [0, 4])
+def test_a_smaller_engine_leaves_the_larger_one_its_shared_memory(cluster_size):
+    from jellyfih_b200 import Engine, InstanceSpec
+    big = Engine([InstanceSpec(2000, 128, 256, 2.0)] * 32, cluster_size=cluster_size)
+    small = Engine([InstanceSpec(500, 32, 32, 1.0)], cluster_size=cluster_size)
+    big.step(3)
+    small.step(3)
+    big.step(3)
+    assert big.sync() and small.sync()
+    big.close()
+    small.close()
