@@ -332,7 +332,7 @@ __device__ __forceinline__ void run_task(const JfEnv<Args>& E, const Win& w, boo
       }
       jf_g2p_advect(I, x, v);
       if (E.do_glow) E.a.glow[k] = jf_glow(E.a.glow[k], jp);
-      nonfinite |= !(isfinite(x.x) && isfinite(x.y) && isfinite(v.x) && isfinite(v.y));
+      nonfinite |= !(isfinite(v.x) && isfinite(v.y));  // the wall clamp leaves x finite whatever it was
       E.a.xv[k] = make_float4(x.x, x.y, v.x, v.y);
       // this pass's P2G takes C from registers and the next pass's G2P
       // recomputes it, so C is stored only by the chunk's last pass and
