@@ -24,6 +24,7 @@ thread_local std::string g_create_err;
 constexpr int kHaloRows = 4;  // batched window rows beyond the band (1 below, 3 above)
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 1024;  // the chunk kernel's static shared variables, rounded up
+constexpr size_t kFramePiece = (size_t)1 << 22;  // pixels a frame read packs at a time: bounds its staging
 constexpr size_t kBandSlackSmem = 128 * 1024;  // window size up to which bands get spare rows
 
 int fail(jf_engine* e, int code, const std::string& msg) {
@@ -114,47 +115,51 @@ int set_live_count(jf_engine* e, int m, int32_t live) {
   return upload_order(e);
 }
 
-// Instance m's particle arrays in engine order, copied to the host.
-struct HostInstance {
-  std::vector<float4> xv, C, F;
-  std::vector<int32_t> mat, slot;
-  std::vector<float2> fiber;
-  std::vector<float> Jp, glow;
-};
-
-int download_instance(jf_engine* e, int m, HostInstance& h) {
-  const JfInst& I = e->inst[m];
-  const size_t n = (size_t)I.n_slots;
-  h.xv.resize(n); h.C.resize(n); h.F.resize(n); h.mat.resize(n); h.slot.resize(n);
-  h.fiber.resize(n); h.Jp.resize(n); h.glow.resize(n);
-  if (n == 0) return JF_OK;
-  const int64_t o = I.p_off;
-  JF_CK(cudaMemcpyAsync(h.xv.data(), e->p.xv + o, n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream), "read xv");
-  JF_CK(cudaMemcpyAsync(h.C.data(), e->p.C + o, n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream), "read C");
-  JF_CK(cudaMemcpyAsync(h.F.data(), e->p.F + o, n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream), "read F");
-  JF_CK(cudaMemcpyAsync(h.mat.data(), e->p.mat + o, n * sizeof(int32_t), cudaMemcpyDeviceToHost, e->stream), "read mat");
-  JF_CK(cudaMemcpyAsync(h.slot.data(), e->p.slot + o, n * sizeof(int32_t), cudaMemcpyDeviceToHost, e->stream), "read slot");
-  JF_CK(cudaMemcpyAsync(h.fiber.data(), e->p.fiber + o, n * sizeof(float2), cudaMemcpyDeviceToHost, e->stream), "read fiber");
-  JF_CK(cudaMemcpyAsync(h.Jp.data(), e->p.Jp + o, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream), "read Jp");
-  JF_CK(cudaMemcpyAsync(h.glow.data(), e->p.glow + o, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream), "read glow");
-  JF_CK(cudaStreamSynchronize(e->stream), "read particles sync");
-  for (size_t k = 0; k < n; ++k) {
-    if (h.slot[k] < 0 || (size_t)h.slot[k] >= n) return fail(e, JF_ERR_CUDA, "corrupt slot permutation");
-  }
+// The staging buffer for frame reads and, on the plain path, slot-order reads
+// and writes: at least `floats` floats, kept with the engine.
+int need_slot_stage(jf_engine* e, size_t floats) {
+  if (e->slot_stage_floats >= floats) return JF_OK;
+  JF_CK(cudaStreamSynchronize(e->stream), "slot staging sync");
+  cudaFree(e->d_slot_stage);
+  e->d_slot_stage = nullptr;
+  e->slot_stage_floats = 0;
+  JF_CK(alloc(&e->d_slot_stage, floats), "cudaMalloc slot staging");
+  e->slot_stage_floats = floats;
   return JF_OK;
 }
 
-int upload_instance(jf_engine* e, int m, const HostInstance& h) {
-  const JfInst& I = e->inst[m];
-  const size_t n = (size_t)I.n_slots;
-  if (n == 0) return JF_OK;
-  const int64_t o = I.p_off;
-  JF_CK(cudaMemcpyAsync(e->p.xv + o, h.xv.data(), n * sizeof(float4), cudaMemcpyHostToDevice, e->stream), "write xv");
-  JF_CK(cudaMemcpyAsync(e->p.C + o, h.C.data(), n * sizeof(float4), cudaMemcpyHostToDevice, e->stream), "write C");
-  JF_CK(cudaMemcpyAsync(e->p.F + o, h.F.data(), n * sizeof(float4), cudaMemcpyHostToDevice, e->stream), "write F");
-  JF_CK(cudaMemcpyAsync(e->p.Jp + o, h.Jp.data(), n * sizeof(float), cudaMemcpyHostToDevice, e->stream), "write Jp");
-  JF_CK(cudaMemcpyAsync(e->p.glow + o, h.glow.data(), n * sizeof(float), cudaMemcpyHostToDevice, e->stream), "write glow");
-  JF_CK(cudaStreamSynchronize(e->stream), "write particles sync");
+// Device arrays for instance m's fields in the caller's (slot) order: the sort's
+// destination buffers, which hold nothing between calls, or on the plain path,
+// which has none, the staging buffer.
+struct SlotArrays {
+  float2 *x, *v;
+  float4 *C, *F;
+  int32_t* mat;
+  float *Jp, *glow;
+  float2* fiber;
+};
+
+int slot_arrays(jf_engine* e, int m, SlotArrays& a) {
+  const size_t n = (size_t)e->inst[m].n_slots;
+  if (e->q.xv) {
+    const int64_t o = e->inst[m].p_off;
+    a = SlotArrays{reinterpret_cast<float2*>(e->q.xv + o), reinterpret_cast<float2*>(e->q.xv + o) + n, e->q.C + o,
+                   e->q.F + o, e->q.mat + o, e->q.Jp + o, e->q.glow + o, e->q.fiber + o};
+    return JF_OK;
+  }
+  // 18 floats a slot, the float4 arrays first so that they stay aligned
+  const int rc = need_slot_stage(e, 18 * n);
+  if (rc) return rc;
+  float* p = e->d_slot_stage;
+  auto take = [&](size_t floats) { float* at = p; p += floats * n; return at; };
+  a.C = reinterpret_cast<float4*>(take(4));
+  a.F = reinterpret_cast<float4*>(take(4));
+  a.x = reinterpret_cast<float2*>(take(2));
+  a.v = reinterpret_cast<float2*>(take(2));
+  a.fiber = reinterpret_cast<float2*>(take(2));
+  a.mat = reinterpret_cast<int32_t*>(take(1));
+  a.Jp = take(1);
+  a.glow = take(1);
   return JF_OK;
 }
 
@@ -448,7 +453,7 @@ int jf_destroy(jf_engine* e) {
   cudaFree(e->d_ep_stats); cudaFree(e->d_grid); cudaFree(e->d_stats); cudaFree(e->d_err);
   cudaFree(e->d_stage); cudaFree(e->d_stage_i); cudaFree(e->d_path);
   cudaFree(e->d_fit); cudaFree(e->d_fit_f); cudaFree(e->d_fit_i); cudaFree(e->d_time);
-  cudaFree(e->d_frame); cudaFree(e->d_vort); cudaFree(e->d_hue);
+  cudaFree(e->d_frame); cudaFree(e->d_vort); cudaFree(e->d_hue); cudaFree(e->d_slot_stage);
   if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
   for (auto& pr : e->step_events) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
   for (auto& pr : e->sort_events) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
@@ -933,15 +938,13 @@ int jf_grad_positions(jf_engine* e, int32_t m, float* dx0) {
                 "jf_grad_positions needs the backward of the latest rollout (jf_grad_backward or jf_grad_step)");
   int rc = set_device(e);
   if (rc) return rc;
-  std::vector<float4> lx;
-  JF_CK(jf_grad_x0_impl(e, m, lx), "read position adjoint");
-  HostInstance h;
-  if ((rc = download_instance(e, m, h))) return rc;
-  for (size_t k = 0; k < lx.size(); ++k) {
-    const size_t s = (size_t)h.slot[k];
-    dx0[2 * s] = lx[k].x;
-    dx0[2 * s + 1] = lx[k].y;
-  }
+  const size_t n = (size_t)e->inst[m].n_slots;
+  if (n == 0) return JF_OK;
+  SlotArrays a;
+  if ((rc = slot_arrays(e, m, a))) return rc;
+  JF_CK(jf_grad_x0_launch(e, m, a.x), "position adjoint");
+  JF_CK(cudaMemcpyAsync(dx0, a.x, sizeof(float2) * n, cudaMemcpyDeviceToHost, e->stream), "read position adjoint");
+  JF_CK(cudaStreamSynchronize(e->stream), "position adjoint sync");
   return JF_OK;
 }
 
@@ -951,20 +954,17 @@ int jf_read_particles(jf_engine* e, int32_t m, float* x, float* v, float* C, flo
   if (m < 0 || m >= e->M) return fail(e, JF_ERR_INVALID, "instance index out of range");
   int rc = set_device(e);
   if (rc) return rc;
-  HostInstance h;
-  if ((rc = download_instance(e, m, h))) return rc;
-  const size_t n = h.slot.size();
-  for (size_t k = 0; k < n; ++k) {
-    const size_t s = (size_t)h.slot[k];
-    if (x) { x[2 * s] = h.xv[k].x; x[2 * s + 1] = h.xv[k].y; }
-    if (v) { v[2 * s] = h.xv[k].z; v[2 * s + 1] = h.xv[k].w; }
-    if (C) { C[4 * s] = h.C[k].x; C[4 * s + 1] = h.C[k].y; C[4 * s + 2] = h.C[k].z; C[4 * s + 3] = h.C[k].w; }
-    if (F) { F[4 * s] = h.F[k].x; F[4 * s + 1] = h.F[k].y; F[4 * s + 2] = h.F[k].z; F[4 * s + 3] = h.F[k].w; }
-    if (material) material[s] = h.mat[k];
-    if (Jp) Jp[s] = h.Jp[k];
-    if (glow) glow[s] = h.glow[k];
-    if (fiber) { fiber[2 * s] = h.fiber[k].x; fiber[2 * s + 1] = h.fiber[k].y; }
-  }
+  const size_t n = (size_t)e->inst[m].n_slots;
+  if (n == 0) return JF_OK;
+  SlotArrays a;
+  if ((rc = slot_arrays(e, m, a))) return rc;
+  JF_CK(jf_slots_out_launch(e, m, a.x, a.v, a.C, a.F, a.mat, a.Jp, a.glow, a.fiber), "slot order");
+  const struct { void* to; const void* from; size_t bytes; } parts[] = {
+      {x, a.x, 8 * n}, {v, a.v, 8 * n}, {C, a.C, 16 * n}, {F, a.F, 16 * n},
+      {material, a.mat, 4 * n}, {Jp, a.Jp, 4 * n}, {glow, a.glow, 4 * n}, {fiber, a.fiber, 8 * n}};
+  for (const auto& p : parts)
+    if (p.to) JF_CK(cudaMemcpyAsync(p.to, p.from, p.bytes, cudaMemcpyDeviceToHost, e->stream), "read particles");
+  JF_CK(cudaStreamSynchronize(e->stream), "read particles sync");
   return JF_OK;
 }
 
@@ -974,19 +974,19 @@ int jf_write_particles(jf_engine* e, int32_t m, const float* x, const float* v, 
   if (m < 0 || m >= e->M) return fail(e, JF_ERR_INVALID, "instance index out of range");
   int rc = set_device(e);
   if (rc) return rc;
-  HostInstance h;
-  if ((rc = download_instance(e, m, h))) return rc;
-  const size_t n = h.slot.size();
-  for (size_t k = 0; k < n; ++k) {
-    const size_t s = (size_t)h.slot[k];
-    if (x) { h.xv[k].x = x[2 * s]; h.xv[k].y = x[2 * s + 1]; }
-    if (v) { h.xv[k].z = v[2 * s]; h.xv[k].w = v[2 * s + 1]; }
-    if (C) h.C[k] = make_float4(C[4 * s], C[4 * s + 1], C[4 * s + 2], C[4 * s + 3]);
-    if (F) h.F[k] = make_float4(F[4 * s], F[4 * s + 1], F[4 * s + 2], F[4 * s + 3]);
-    if (Jp) h.Jp[k] = Jp[s];
-    if (glow) h.glow[k] = glow[s];
+  const size_t n = (size_t)e->inst[m].n_slots;
+  if (n > 0) {
+    SlotArrays a;
+    if ((rc = slot_arrays(e, m, a))) return rc;
+    const struct { const float* from; void* to; size_t bytes; } parts[] = {
+        {x, a.x, 8 * n}, {v, a.v, 8 * n}, {C, a.C, 16 * n}, {F, a.F, 16 * n}, {Jp, a.Jp, 4 * n}, {glow, a.glow, 4 * n}};
+    for (const auto& p : parts)
+      if (p.from) JF_CK(cudaMemcpyAsync(p.to, p.from, p.bytes, cudaMemcpyHostToDevice, e->stream), "write particles");
+    JF_CK(jf_slots_in_launch(e, m, x ? a.x : nullptr, v ? a.v : nullptr, C ? a.C : nullptr, F ? a.F : nullptr,
+                             Jp ? a.Jp : nullptr, glow ? a.glow : nullptr),
+          "engine order");
+    JF_CK(cudaStreamSynchronize(e->stream), "write particles sync");
   }
-  if ((rc = upload_instance(e, m, h))) return rc;
   if (x) e->sorted = false;
   return JF_OK;
 }
@@ -1111,6 +1111,7 @@ int jf_frame_create(jf_engine* e, int32_t video_res) {
     e->frame_res = 0;
     JF_CK(alloc(&e->d_frame, (size_t)video_res * video_res), "cudaMalloc frame");
     e->frame_res = video_res;
+    if ((rc = need_slot_stage(e, 3 * std::min((size_t)video_res * video_res, kFramePiece)))) return rc;
   }
   JF_CK(cudaMemsetAsync(e->d_frame, 0, sizeof(float4) * (size_t)video_res * video_res, e->stream), "clear frame");
   return JF_OK;
@@ -1188,14 +1189,15 @@ int jf_read_frame(jf_engine* e, float* rgb) {
   int rc = set_device(e);
   if (rc) return rc;
   const size_t n = (size_t)e->frame_res * e->frame_res;
-  std::vector<float4> f(n);
-  JF_CK(cudaMemcpyAsync(f.data(), e->d_frame, sizeof(float4) * n, cudaMemcpyDeviceToHost, e->stream), "read frame");
-  JF_CK(cudaStreamSynchronize(e->stream), "read frame sync");
-  for (size_t k = 0; k < n; ++k) {
-    rgb[3 * k] = f[k].x;
-    rgb[3 * k + 1] = f[k].y;
-    rgb[3 * k + 2] = f[k].z;
+  const size_t piece = std::min(n, kFramePiece);
+  if ((rc = need_slot_stage(e, 3 * piece))) return rc;
+  for (size_t at = 0; at < n; at += piece) {
+    const size_t m = std::min(piece, n - at);
+    JF_CK(jf_frame_pack_launch(e, (int64_t)at, (int64_t)m, e->d_slot_stage), "pack frame");
+    JF_CK(cudaMemcpyAsync(rgb + 3 * at, e->d_slot_stage, sizeof(float) * 3 * m, cudaMemcpyDeviceToHost, e->stream),
+          "read frame");
   }
+  JF_CK(cudaStreamSynchronize(e->stream), "read frame sync");
   return JF_OK;
 }
 

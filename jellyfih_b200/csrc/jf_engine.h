@@ -81,6 +81,8 @@ struct jf_engine {
   int32_t* d_err = nullptr;        // per-instance non-finite flags
   float* d_stage = nullptr;        // host <-> device staging (max_slots * 8 floats)
   int32_t* d_stage_i = nullptr;    // staging for ints (max_slots * 2)
+  float* d_slot_stage = nullptr;   // packed frames; plain path: slot-order reads and writes
+  size_t slot_stage_floats = 0;
   unsigned long long* d_path = nullptr;  // batched path counters (see jf_path_counts)
   double* d_fit = nullptr;         // fitness staging: M x 5 rows + M scores
   double* d_fit_f = nullptr;       // fitness staging: M contraction genes
@@ -164,7 +166,8 @@ cudaError_t jf_grad_forward_impl(jf_engine* e, int64_t steps, int32_t K, const i
 cudaError_t jf_grad_backward_impl(jf_engine* e, double* gparam_host);
 cudaError_t jf_grad_step_impl(jf_engine* e, int64_t steps, int32_t K, const int32_t* body_mode,
                               const double* inv_n, double* gparam_host);
-cudaError_t jf_grad_x0_impl(jf_engine* e, int m, std::vector<float4>& out);
+// Position adjoint of instance m's initial state, in slot order.
+cudaError_t jf_grad_x0_launch(jf_engine* e, int m, float2* d_out);
 bool jf_grad_done(const jf_engine* e, int stage);
 void jf_grad_free(jf_engine* e);
 // The rollout's loss sums into e->d_stats (from the FP64 final state in the FP64 build).
@@ -174,6 +177,12 @@ cudaError_t jf_grad_loss_stats(jf_engine* e);
 cudaError_t jf_stats_launch(jf_engine* e);
 
 // Kernels used by the C-ABI for loading, reading and writing particles.
+// Instance m's fields between engine order and slot order (device arrays;
+// nullptr fields of an import are left as they are).
+cudaError_t jf_slots_out_launch(jf_engine* e, int m, float2* x, float2* v, float4* C, float4* F, int32_t* mat,
+                                float* Jp, float* glow, float2* fiber);
+cudaError_t jf_slots_in_launch(jf_engine* e, int m, const float2* x, const float2* v, const float4* C,
+                               const float4* F, const float* Jp, const float* glow);
 cudaError_t jf_load_launch(jf_engine* e, int m, int32_t n);
 // Copies instance m's glow into slot order at d_stage + 4 * max_slots.
 cudaError_t jf_glow_to_slot_order(jf_engine* e, int m);
@@ -186,6 +195,8 @@ cudaError_t jf_render_overlay_launch(jf_engine* e, int res_sub, int grid_side, f
 cudaError_t jf_vorticity_launch(jf_engine* e, float scale);
 cudaError_t jf_render_vort_launch(jf_engine* e, int res_sub, int grid_side, float alpha, int style);
 cudaError_t jf_tone_map_launch(jf_engine* e);
+// Pixels first .. first + n - 1 of the frame as n x 3 floats.
+cudaError_t jf_frame_pack_launch(jf_engine* e, int64_t first, int64_t n, float* d_rgb);
 // Tank fill (jf_tank.cu): water lattice of instance m minus the robot's
 // margin, placed after the robot in the load staging; *h_total = kept
 // candidates (read back on the engine's stream; valid after a sync).

@@ -1412,19 +1412,23 @@ cudaError_t step_impl(jf_engine* e, int64_t steps, int32_t K, const int32_t* bod
   return err;
 }
 
+// Position adjoint of instance I in slot order, rounded to FP32.
 template <class R>
-cudaError_t x0_impl(jf_engine* e, int m, std::vector<float4>& out) {
+__global__ void x0_kernel(JfInst I, const V4<R>* __restrict__ lxv, const int32_t* __restrict__ slot,
+                          float2* __restrict__ out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= I.n_slots) return;
+  const int64_t g = I.p_off + k;
+  const V4<R> a = lxv[g];
+  out[slot[g]] = make_float2((float)a.x, (float)a.y);
+}
+
+template <class R>
+cudaError_t x0_launch(jf_engine* e, int m, float2* d_out) {
   const JfInst& I = e->inst[m];
-  out.resize((size_t)I.n_slots);
-  if (I.n_slots == 0) return cudaSuccess;
-  std::vector<V4<R>> tmp((size_t)I.n_slots);
-  cudaError_t err = cudaMemcpyAsync(tmp.data(), bufs<R>(e).lxv + I.p_off, sizeof(V4<R>) * I.n_slots,
-                                    cudaMemcpyDeviceToHost, e->stream);
-  if (err != cudaSuccess) return err;
-  if ((err = cudaStreamSynchronize(e->stream))) return err;
-  for (size_t k = 0; k < tmp.size(); ++k)
-    out[k] = make_float4((float)tmp[k].x, (float)tmp[k].y, (float)tmp[k].z, (float)tmp[k].w);
-  return cudaSuccess;
+  x0_kernel<R><<<(I.n_slots + kT - 1) / kT, kT, 0, e->stream>>>(I, bufs<R>(e).lxv, e->p.slot, d_out);
+  e->launches += 1;
+  return cudaGetLastError();
 }
 
 bool fp64(const jf_engine* e) { return (e->flags & JF_FLAG_GRAD_FP64) != 0; }
@@ -1453,9 +1457,9 @@ cudaError_t jf_grad_step_impl(jf_engine* e, int64_t steps, int32_t K, const int3
                  : step_impl<float>(e, steps, K, body_mode, inv_n, gparam_host);
 }
 
-// Position adjoint of the initial state for one instance, in engine order.
-cudaError_t jf_grad_x0_impl(jf_engine* e, int m, std::vector<float4>& out) {
-  return fp64(e) ? x0_impl<double>(e, m, out) : x0_impl<float>(e, m, out);
+// Position adjoint of the initial state for one instance, in slot order.
+cudaError_t jf_grad_x0_launch(jf_engine* e, int m, float2* d_out) {
+  return fp64(e) ? x0_launch<double>(e, m, d_out) : x0_launch<float>(e, m, d_out);
 }
 
 // Whether the engine's latest rollout completed its forward (stage 1) or its
