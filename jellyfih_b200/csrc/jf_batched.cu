@@ -620,8 +620,10 @@ __global__ void dead_glow_kernel(const JfInst* __restrict__ inst, const int32_t*
   }
 }
 
-// sim_time += dt, K times, as the FP32 running sum of mpm_sim.py:340
-__global__ void advance_time_kernel(float* t, int K, float dt) {
+// sim_time += dt, K times, as the FP32 running sum of mpm_sim.py:340, and the
+// spans' substep counter
+__global__ void advance_time_kernel(float* t, int K, float dt, uint32_t* tag, uint32_t tag_step) {
+  if (tag) *tag += tag_step;
   float v = *t;
   for (int s = 0; s < K; ++s) v = v + dt;
   *t = v;
@@ -769,7 +771,8 @@ static cudaError_t chunk_with_sort(jf_engine* e, int K) {
   cudaError_t err = jf_batched_sort(e);
   if (err != cudaSuccess) return err;
   if ((err = launch_chunk(e, K)) != cudaSuccess) return err;
-  advance_time_kernel<<<1, 1, 0, e->stream>>>(e->d_time, K, (float)e->dt);
+  advance_time_kernel<<<1, 1, 0, e->stream>>>(e->d_time, K, (float)e->dt, e->span ? jf_span_tag(e) : nullptr,
+                                             e->span ? jf_span_tag_step(e, K) : 0u);
   e->launches += 1;
   e->sorted = false;  // particles moved: re-sort before the next chunk
   return cudaGetLastError();

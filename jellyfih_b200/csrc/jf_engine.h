@@ -149,6 +149,8 @@ cudaError_t jf_span_setup(jf_engine* e, int threads);
 cudaError_t jf_span_sort(jf_engine* e);
 cudaError_t jf_span_launch(jf_engine* e, int K);
 void jf_span_free(jf_engine* e);
+uint32_t* jf_span_tag(const jf_engine* e);
+uint32_t jf_span_tag_step(const jf_engine* e, int K);
 
 // Episode helpers (jf_run_episode): load every instance from slot-ordered
 // staging, and the (M, 5) rows from before / after CoM sums, on the device.

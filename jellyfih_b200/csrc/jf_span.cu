@@ -16,17 +16,19 @@
 // s (mpm_sim.py:312-333 then :168-271).  Neighbouring bands of an instance
 // overlap in the four rows around their cut (the stencil's reach plus one row
 // of drift either way).  After a pass each side writes its partial sums of
-// those rows to global memory, the instance's CTAs meet at a counter, and each
-// side adds the other's sums and updates the rows for itself: the same two
-// terms, so the same bits, and one meeting per substep.  The rows between are
-// updated while the counters travel.
+// those rows to global memory and takes the other's, and updates the rows for
+// itself: the same two terms, so the same bits.  A node travels as one 16-byte
+// word of its sums and the substep's tag, written and read whole, so that the
+// reader polls the data itself and no fence stands in its way.  Beside it the
+// instance's CTAs count their arrivals, which keeps them within a substep of
+// one another.  The rows between are updated while the words travel.
 //
 // A particle whose stencil has drifted out of its CTA's window (more than a
-// row since the last re-sort) adds to a spill grid in global memory and raises
-// the instance's drift flag of that substep; the instance's CTAs then add the
-// spill to their rows, publish their updated rows and meet a second time, so
-// that the particle can gather them in the next pass.  The result does not
-// depend on the re-sort interval.
+// row since the last re-sort) adds to a spill grid in global memory, and its
+// CTA's arrival carries a drift mark; the instance's CTAs then add the spill to
+// their rows, publish their updated rows and meet a second time, so that the
+// particle can gather them in the next pass.  The result does not depend on
+// the re-sort interval.
 //
 // Every wait counts its polls and gives up after kSpinLimit: the CTA raises
 // the abort flag, which ends the waits of the others, frees its tensor memory
@@ -83,7 +85,6 @@ struct JfSpan {
   std::vector<SpanGroup> groups;
   int32_t threads = 0;     // threads of a CTA
   int32_t n_cta = 0;       // CTAs of a launch (table stride)
-  int32_t nx_max = 0;
   int32_t total_rows = 0;
   int32_t cap_nodes = 0;   // window nodes of a CTA
   size_t smem = 0;
@@ -97,11 +98,15 @@ struct JfSpan {
   int4* d_seg = nullptr;          // groups x n_cta x kMaxSeg: (instance, first row, end row, 0)
   int32_t* d_nseg = nullptr;      // groups x n_cta
   int32_t* d_nbar = nullptr;      // M: CTAs that hold a band of the instance
-  uint32_t* d_bar = nullptr;      // 2 M: arrivals at the substep's meeting, at the drift meeting
-  int32_t* d_drift = nullptr;     // 3 M: drift flag of a substep (mod 3)
+  // 3 M: arrivals of even and of odd substeps (drift marks in the upper half), of drift meetings
+  unsigned long long* d_bar = nullptr;
+  int32_t* d_drift = nullptr;     // M: bit s % 3: the spill grid of substep s is in use
+  uint32_t* d_tag = nullptr;      // tag of the next chunk's first substep
   int32_t* d_abort = nullptr;
   float4* d_spill = nullptr;      // 3 x total nodes
-  float4* d_slot = nullptr;       // n_cta x 2 sides x 2 parities x kOverlap x nx_max
+  // n_cta x 2 sides x 2 parities x kOverlap x nx_max nodes (twice that, the hoop
+  // sums in the second half, in the axisymmetric variant)
+  uint4* d_slot = nullptr;
 };
 
 namespace {
@@ -127,18 +132,19 @@ struct SpanArgs {
   const int4* seg;            // of this group
   const int32_t* nseg;
   const int32_t* nbar;
-  uint32_t* bar;
+  unsigned long long* bar;
   int32_t* drift;
   int32_t* abort;
+  const uint32_t* tag;        // counter of the substeps run so far
+  uint32_t tag_add;           // of the groups launched before this one in the chunk
   float4* spill;
-  float4* slot;
+  uint4* slot;
   float4* grid;               // grid of the chunk's last substep, node = g_off + j * nx + i
   int32_t* err;
   unsigned long long* path;
   const float* t_dev;
   int64_t nodes;              // nodes of all instances (stride of the spill grids)
   int32_t M;
-  int32_t nx_max;
   int32_t stride;
   int32_t K;
   float dt;
@@ -154,6 +160,8 @@ struct SpanSeg {
   int cap;
   int n_bar;             // CTAs of the instance
   int n_meet2;           // drift meetings so far
+  int drifted;           // this CTA scattered into the spill grid in the current pass
+  unsigned marks[2];     // drift marks of even and odd substeps so far
   int ov_beg, n_ov;      // its part of the overflow list
   int oor_beg, n_oor;    // live particles outside every stencil range (the instance's last band takes them)
   int gen0, n_gen;       // generic tasks: first, count
@@ -169,37 +177,66 @@ struct SpanSeg {
 // grid and the spill grid.
 struct SpanWindow : JfWindow {
   const SpanArgs& a;
-  const SpanSeg& S;
+  SpanSeg& S;
   const int& s;  // the substep
   __device__ __forceinline__ float2 far_gather(int i, int j) const {
     const float4 g = __ldcg(a.grid + S.I.g_off + (int64_t)j * S.I.nx + i);
     return make_float2(g.x, g.y);
   }
   __device__ __forceinline__ void far_scatter(int i, int j, float3 c, float h, bool) const {
-    const int r = s % 3;
-    atomicAdd(a.spill + r * a.nodes + S.I.g_off + (int64_t)j * S.I.nx + i, make_float4(c.x, c.y, c.z, h));
-    *(volatile int32_t*)(a.drift + 3 * S.m + r) = 1;
+    atomicAdd(a.spill + (s % 3) * a.nodes + S.I.g_off + (int64_t)j * S.I.nx + i, make_float4(c.x, c.y, c.z, h));
+    *(volatile int*)&S.drifted = 1;
   }
 };
 
-__device__ __forceinline__ void arrive(uint32_t* p) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+constexpr unsigned long long kMark = 1ull << 40;  // a drift mark in an arrival count
+
+__device__ __forceinline__ void arrive(unsigned long long* p, unsigned long long n) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(n) : "memory");
 }
 
-// Waits until *p has reached `target` (counters only grow within a launch);
-// false when the wait gave up or another CTA did.
-__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t target, int32_t* abort) {
-  for (unsigned n = 0; n < kSpinLimit; ++n) {
-    uint32_t v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    if ((int32_t)(v - target) >= 0) {
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      return true;
-    }
-    if ((n & 63u) == 63u && *(volatile int32_t*)abort != 0) return false;
+// One poll of a wait; false when the wait gave up or another CTA did.
+__device__ __forceinline__ bool keep_polling(unsigned& n, int32_t* abort) {
+  if (++n >= kSpinLimit) {
+    atomicExch(abort, 1);
+    return false;
   }
-  atomicExch(abort, 1);
-  return false;
+  return (n & 63u) != 0u || *(volatile int32_t*)abort == 0;
+}
+
+// Waits until the arrivals at *p have reached `target` (they only grow within a
+// launch); *seen is the count with its marks.
+__device__ __forceinline__ bool wait_for(const unsigned long long* p, unsigned long long target, int32_t* abort,
+                                         unsigned long long* seen) {
+  for (unsigned n = 0;;) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    *seen = v;
+    if ((v & (kMark - 1)) >= target) return true;
+    if (!keep_polling(n, abort)) return false;
+  }
+}
+
+// A 16-byte word written and read as one access: three values and a tag.
+__device__ __forceinline__ void send(uint4* p, float a, float b, float c, uint32_t tag) {
+  asm volatile(
+      "{\n\t.reg .b128 w;\n\t.reg .b64 l, h;\n\tmov.b64 l, {%1, %2};\n\tmov.b64 h, {%3, %4};\n\t"
+      "mov.b128 w, {l, h};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
+      "f"(a), "f"(b), "f"(c), "r"(tag)
+      : "memory");
+}
+__device__ __forceinline__ bool receive(const uint4* p, uint32_t tag, int32_t* abort, float3* v) {
+  for (unsigned n = 0;;) {
+    uint32_t t;
+    asm volatile(
+        "{\n\t.reg .b128 w;\n\t.reg .b64 l, h;\n\tld.relaxed.gpu.global.b128 w, [%4];\n\tmov.b128 {l, h}, w;\n\t"
+        "mov.b64 {%0, %1}, l;\n\tmov.b64 {%2, %3}, h;\n\t}"
+        : "=f"(v->x), "=f"(v->y), "=f"(v->z), "=r"(t)
+        : "l"(p)
+        : "memory");
+    if (t == tag) return true;
+    if (!keep_polling(n, abort)) return false;
+  }
 }
 
 // kTmem: the node blocks live in TMEM (544 .. 768 threads); otherwise in
@@ -236,6 +273,8 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
     S.cap = a.cap[q.x];
     S.n_bar = a.nbar[q.x];
     S.n_meet2 = 0;
+    S.drifted = 0;
+    S.marks[0] = S.marks[1] = 0u;
     const int32_t* ovr = a.ovrow + a.rowoff[q.x] + q.x;
     S.ov_beg = ovr[q.y];
     S.n_ov = ovr[q.z] - S.ov_beg;
@@ -252,6 +291,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
   if (tid < 4) s_path[tid] = 0u;
   __syncthreads();
   float t = *a.t_dev;
+  const uint32_t tag0 = *a.tag + a.tag_add;
   if (tid == 0) {
     int gen = 0, cell = 0, off = 0;
     for (int q = 0; q < nseg; ++q) {
@@ -294,7 +334,8 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
   for (int n = tid; n < (kAxisym ? 6 : 5) * WN; n += nth) reinterpret_cast<float*>(smem4)[n] = 0.0f;
   __syncthreads();
 
-  const int64_t slot_n = (int64_t)kOverlap * a.nx_max;
+  const int nx = a.I.nx;
+  const int64_t slot_n = (int64_t)kOverlap * nx * (kAxisym ? 2 : 1), slot_half = (int64_t)kOverlap * nx;
 
   for (int s = 0; s <= a.K; ++s) {
     const bool do_g2p = s > 0;
@@ -310,7 +351,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
       } else {
         while (q + 1 < nseg && task - n_gen >= s_seg[q + 1].cell0) ++q;
       }
-      const SpanSeg& S = s_seg[q];
+      SpanSeg& S = s_seg[q];
       // kernel parameters where the instances agree: operands of the arithmetic that take no registers
       JfInst I = a.I;
       I.axisym = kAxisym;
@@ -353,110 +394,125 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
     }
     __syncthreads();
     if (!do_p2g) break;
-    float4* const spill = a.spill + (int64_t)(s % 3) * a.nodes;
-
+    const uint32_t tag = tag0 + (uint32_t)s;
+    if (tid < nseg) {
+      SpanSeg& S = s_seg[tid];
+      if (S.n_bar > 1) {
+        unsigned long long n = 1;
+        // the spill is there for whoever sees the mark, and rows cleared in the
+        // substep before are clear for the next to use that grid
+        if (S.drifted || s_drift[s & 1][tid]) __threadfence();
+        if (S.drifted) {
+          S.drifted = 0;
+          atomicOr(a.drift + S.m, 1 << (s % 3));
+          n += kMark;
+        }
+        arrive(a.bar + (s & 1) * a.M + S.m, n);
+      }
+    }
     // partial sums of the rows around the cuts, for the other side
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
       const SpanSeg& S = s_seg[side ? nseg - 1 : 0];
       if (!(side ? S.upper() : S.lower())) continue;
-      const int n0 = S.off + (side ? S.hi - S.lo : 0) * S.I.nx;
-      float4* const to = a.slot + ((cta * 2 + side) * 2 + (s & 1)) * slot_n;
-      for (int n = tid; n < kOverlap * S.I.nx; n += nth)
-        __stcg(to + n, make_float4(Ax[n0 + n], Ay[n0 + n], Am[n0 + n], kAxisym ? Ah[n0 + n] : 0.0f));
+      const int n0 = S.off + (side ? S.hi - S.lo : 0) * nx;
+      uint4* const to = a.slot + ((cta * 2 + side) * 2 + (s & 1)) * slot_n;
+      for (int n = tid; n < kOverlap * nx; n += nth) {
+        send(to + n, Ax[n0 + n], Ay[n0 + n], Am[n0 + n], tag);
+        if (kAxisym) send(to + slot_half + n, Ah[n0 + n], 0.0f, 0.0f, tag);
+      }
     }
-    __syncthreads();
-    if (tid < nseg && s_seg[tid].n_bar > 1) arrive(a.bar + s_seg[tid].m);
+    // the next substep's pressures, by the last warp while the words travel
+    t = t + a.dt;
+    if (tid >= nth - 32 && lane < nseg)
+      s_pressure[(s + 1) & 1][lane] =
+          s_seg[lane].P.actuation * jf_activation(s_seg[lane].P.freq, s_seg[lane].P.contraction, t);
 
-    // grid update of one node of band S from its sums; `own`: the band writes
-    // it to the grid in global memory where asked to
+    // grid update of one node of band S from its sums; `publish`: into global
+    // memory too
     const bool last = (s == a.K - 1);
     auto update_node = [&](const SpanSeg& S, int wr, int i, float mx, float my, float mm, float mh, bool publish) {
       const int j = S.lo - kHaloLo + wr;
       const float2 u = jf_grid_node(S.I, i, j, mx, my, mm, mh);
-      G[S.off + wr * S.I.nx + i] = u;
-      if (publish) a.grid[S.I.g_off + (int64_t)j * S.I.nx + i] = make_float4(u.x, u.y, mm, 0.0f);
+      G[S.off + wr * nx + i] = u;
+      if (publish) a.grid[S.I.g_off + (int64_t)j * nx + i] = make_float4(u.x, u.y, mm, 0.0f);
     };
-    // rows that no neighbour shares, while the counters travel.  Their sums
-    // stay until the meeting is over: a spill may come in.
+    // Rows that no neighbour shares, then the rows around the cuts from both
+    // sides' sums.  The sums stay until the meeting is over: a spill may come in.
     for (int q = 0; q < nseg; ++q) {
       const SpanSeg& S = s_seg[q];
-      const int nx = S.I.nx;
       const int n0 = S.in_lo() * nx, n1 = S.in_hi() * nx;
       for (int n = n0 + tid; n < n1; n += nth) {
         const int wr = n / nx, o = S.off + n;
         update_node(S, wr, n - wr * nx, Ax[o], Ay[o], Am[o], kAxisym ? Ah[o] : 0.0f, last);
       }
     }
-    if (tid < nseg) {
-      const SpanSeg& S = s_seg[tid];
-      if (S.n_bar > 1) {
-        if (!wait_for(a.bar + S.m, (uint32_t)(s + 1) * S.n_bar, a.abort)) {
-          s_tot[3] = 1;
-          atomicOr(a.err + S.m, kJfErrAbort);
-        }
-        s_drift[s & 1][tid] = *(volatile int32_t*)(a.drift + 3 * S.m + s % 3);
-      }
-    }
-    __syncthreads();
-    if (s_tot[3]) break;
-
-    // rows around the cuts: both sides' sums, and the spill
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
-      const int q = side ? nseg - 1 : 0;
-      const SpanSeg& S = s_seg[q];
+      const SpanSeg& S = s_seg[side ? nseg - 1 : 0];
       if (!(side ? S.upper() : S.lower())) continue;
-      const int nx = S.I.nx;
       const int wr0 = side ? S.hi - S.lo : 0;
-      const bool drift = s_drift[s & 1][q] != 0;
       const int other = side ? cta + 1 : cta - 1;
-      const float4* const from = a.slot + ((other * 2 + (side ^ 1)) * 2 + (s & 1)) * slot_n;
+      const uint4* const from = a.slot + ((other * 2 + (side ^ 1)) * 2 + (s & 1)) * slot_n;
       for (int n = tid; n < kOverlap * nx; n += nth) {
         const int r = n / nx, i = n - r * nx;
         const int o = S.off + wr0 * nx + n;
-        const float4 b = __ldcg(from + n);
-        float mx = Ax[o] + b.x, my = Ay[o] + b.y, mm = Am[o] + b.z, mh = kAxisym ? Ah[o] + b.w : 0.0f;
-        if (drift) {
-          const float4 e = __ldcg(spill + S.I.g_off + (int64_t)(S.lo - kHaloLo + wr0 + r) * nx + i);
-          mx += e.x;
-          my += e.y;
-          mm += e.z;
-          mh += e.w;
+        float3 b, h = make_float3(0.0f, 0.0f, 0.0f);
+        if (!receive(from + n, tag, a.abort, &b) || (kAxisym && !receive(from + slot_half + n, tag, a.abort, &h))) {
+          s_tot[3] = 1;
+          atomicOr(a.err + S.m, kJfErrAbort);
+          break;
         }
-        const bool own = side ? r == 0 : r > 0;
-        update_node(S, wr0 + r, i, mx, my, mm, mh, own && (last || drift));
-        Ax[o] = 0.0f;
-        Ay[o] = 0.0f;
-        Am[o] = 0.0f;
-        if (kAxisym) Ah[o] = 0.0f;
+        // both sides' sums, kept for a spill
+        const float mx = Ax[o] + b.x, my = Ay[o] + b.y, mm = Am[o] + b.z;
+        const float mh = kAxisym ? Ah[o] + h.x : 0.0f;
+        Ax[o] = mx;
+        Ay[o] = my;
+        Am[o] = mm;
+        if (kAxisym) Ah[o] = mh;
+        update_node(S, wr0 + r, i, mx, my, mm, mh, last && (side ? r == 0 : r > 0));
       }
     }
-    // the other rows: the spill where there is one, and clear sums
+    if (tid < nseg) {
+      SpanSeg& S = s_seg[tid];
+      int drift = 0;
+      if (S.n_bar > 1) {
+        unsigned long long seen;
+        if (!wait_for(a.bar + (s & 1) * a.M + S.m, (unsigned long long)(s / 2 + 1) * S.n_bar, a.abort, &seen)) {
+          s_tot[3] = 1;
+          atomicOr(a.err + S.m, kJfErrAbort);
+        }
+        const unsigned marks = (unsigned)(seen >> 40);
+        drift = marks != S.marks[s & 1];
+        S.marks[s & 1] = marks;
+        if (drift || s_drift[0][tid] || s_drift[1][tid]) __threadfence();
+      }
+      s_drift[s & 1][tid] = drift;
+    }
+    if (tid == 0) s_next_task[(s + 1) & 1] = n_warps;
+    __syncthreads();
+    if (s_tot[3]) break;
+
+    // the spill of this substep where there is one
     bool any_drift = false;
     for (int q = 0; q < nseg; ++q) {
       const SpanSeg& S = s_seg[q];
-      const int nx = S.I.nx;
-      const bool drift = s_drift[s & 1][q] != 0;
-      any_drift |= drift;
-      const int n0 = S.in_lo() * nx, n1 = S.in_hi() * nx;
-      for (int n = n0 + tid; n < n1; n += nth) {
-        const int o = S.off + n;
-        if (drift) {
-          const int wr = n / nx, i = n - wr * nx;
-          const float4 e = __ldcg(spill + S.I.g_off + (int64_t)(S.lo - kHaloLo + wr) * nx + i);
-          update_node(S, wr, i, Ax[o] + e.x, Ay[o] + e.y, Am[o] + e.z, kAxisym ? Ah[o] + e.w : 0.0f, true);
+      const int rows = S.hi - S.lo;
+      if (s_drift[s & 1][q]) {
+        any_drift = true;
+        const int n0 = max(kHaloLo - S.lo, 0) * nx, n1 = min(rows + kHalo, S.I.ny - S.lo + kHaloLo) * nx;
+        for (int n = n0 + tid; n < n1; n += nth) {
+          const int wr = n / nx, i = n - wr * nx, o = S.off + n;
+          const float4 e = __ldcg(a.spill + (s % 3) * a.nodes + S.I.g_off + (int64_t)(S.lo - kHaloLo + wr) * nx + i);
+          update_node(S, wr, i, Ax[o] + e.x, Ay[o] + e.y, Am[o] + e.z, kAxisym ? Ah[o] + e.w : 0.0f,
+                      wr >= kHaloLo && wr < kHaloLo + rows);
         }
-        Ax[o] = 0.0f;
-        Ay[o] = 0.0f;
-        Am[o] = 0.0f;
-        if (kAxisym) Ah[o] = 0.0f;
       }
       // the spill of the substep before has been read by everyone: its rows are cleared by their owners
       if (s > 0 && s_drift[(s - 1) & 1][q]) {
-        float4* const old = a.spill + (int64_t)((s - 1) % 3) * a.nodes + S.I.g_off + (int64_t)S.lo * nx;
-        for (int n = tid; n < (S.hi - S.lo) * nx; n += nth) __stcg(old + n, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-        if (tid == 0 && S.lo == 0) *(volatile int32_t*)(a.drift + 3 * S.m + (s - 1) % 3) = 0;
+        float4* const old = a.spill + ((s - 1) % 3) * a.nodes + S.I.g_off + (int64_t)S.lo * nx;
+        for (int n = tid; n < rows * nx; n += nth) __stcg(old + n, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+        if (tid == 0 && S.lo == 0) atomicAnd(a.drift + S.m, ~(1 << ((s - 1) % 3)));
       }
     }
     if (any_drift) {  // the published rows are there for everyone after a second meeting
@@ -464,18 +520,18 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
       if (tid < nseg && s_drift[s & 1][tid]) {
         SpanSeg& S = s_seg[tid];
         S.n_meet2 += 1;
-        arrive(a.bar + a.M + S.m);
-        if (!wait_for(a.bar + a.M + S.m, (uint32_t)S.n_meet2 * S.n_bar, a.abort)) {
+        __threadfence();
+        arrive(a.bar + 2 * a.M + S.m, 1);
+        unsigned long long seen;
+        if (!wait_for(a.bar + 2 * a.M + S.m, (unsigned long long)S.n_meet2 * S.n_bar, a.abort, &seen)) {
           s_tot[3] = 1;
           atomicOr(a.err + S.m, kJfErrAbort);
         }
+        __threadfence();
       }
     }
-    t = t + a.dt;
-    if (tid < nseg)
-      s_pressure[(s + 1) & 1][tid] =
-          s_seg[tid].P.actuation * jf_activation(s_seg[tid].P.freq, s_seg[tid].P.contraction, t);
-    if (tid == 0) s_next_task[(s + 1) & 1] = n_warps;
+    // clear sums for the next pass
+    for (int n = tid; n < (kAxisym ? 4 : 3) * WN; n += nth) Ax[n] = 0.0f;
     __syncthreads();
     if (any_drift && s_tot[3]) break;
   }
@@ -499,7 +555,8 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
     const JfInst* __restrict__ inst, int32_t* __restrict__ counts, int stride, const int32_t* __restrict__ solid,
     const int32_t* __restrict__ rowoff, int32_t* __restrict__ rowcost, int32_t* __restrict__ ovrow,
     int32_t* __restrict__ ovcur, int32_t* __restrict__ cap_out, int fixed_cap, int32_t* __restrict__ band, int CS,
-    uint32_t* __restrict__ bar, int32_t* __restrict__ drift, int32_t* __restrict__ abort, float4* __restrict__ spill,
+    unsigned long long* __restrict__ bar, int32_t* __restrict__ drift, int32_t* __restrict__ abort,
+    float4* __restrict__ spill,
     int64_t nodes, int M) {
   constexpr int kWarps = kScanThreads / 32;
   __shared__ int s_cost[32];
@@ -515,7 +572,7 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
   const int segs = (I.nx + 31) >> 5;
   // what a chunk's last substeps may have left in the spill grids
   for (int r = 0; r < 3; ++r)
-    if (drift[3 * m + r])
+    if (drift[m] >> r & 1)
       for (int n = tid; n < I.nx * I.ny; n += kScanThreads)
         spill[(int64_t)r * nodes + I.g_off + n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (tid < 32) s_cost[tid] = 0;
@@ -524,8 +581,8 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
     s_row_over[y] = 0;
   }
   __syncthreads();
-  if (tid < 3) drift[3 * m + tid] = 0;
-  if (tid < 2) bar[tid * M + m] = 0u;
+  if (tid == 0) drift[m] = 0;
+  if (tid < 3) bar[tid * M + m] = 0ull;
   if (tid == 0 && m == 0) *abort = 0;
 
   // lane k sums the cost of candidate k (0 = no cap), in quarter lane-iterations
@@ -837,7 +894,7 @@ void jf_span_free(jf_engine* e) {
   if (!s) return;
   cudaFree(s->d_groups); cudaFree(s->d_rowoff); cudaFree(s->d_rowcost); cudaFree(s->d_rowpre); cudaFree(s->d_ovrow);
   cudaFree(s->d_ovcur); cudaFree(s->d_fallback); cudaFree(s->d_seg); cudaFree(s->d_nseg); cudaFree(s->d_nbar);
-  cudaFree(s->d_bar); cudaFree(s->d_drift); cudaFree(s->d_abort); cudaFree(s->d_spill); cudaFree(s->d_slot);
+  cudaFree(s->d_bar); cudaFree(s->d_drift); cudaFree(s->d_abort); cudaFree(s->d_tag); cudaFree(s->d_spill); cudaFree(s->d_slot);
   delete s;
   e->span = nullptr;
 }
@@ -920,23 +977,26 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
   s->threads = threads;
   s->groups = groups;
   s->n_cta = n_cta;
-  s->nx_max = nx_max;
   s->total_rows = rowoff[e->M];
   s->cap_nodes = (int32_t)cap;
   s->smem = smem;
+  const size_t slots = (size_t)n_cta * 4 * kOverlap * nx_max * ((e->flags & JF_FLAG_AXISYM) ? 2 : 1);
   const size_t ng = groups.size(), rows = (size_t)s->total_rows, M = (size_t)e->M;
   if ((err = dev(&s->d_groups, ng)) || (err = dev(&s->d_rowoff, M + 1)) || (err = dev(&s->d_rowcost, rows)) ||
       (err = dev(&s->d_rowpre, rows)) || (err = dev(&s->d_ovrow, rows + M)) || (err = dev(&s->d_ovcur, rows)) ||
       (err = dev(&s->d_fallback, table.size())) || (err = dev(&s->d_seg, ng * n_cta * kMaxSeg)) ||
-      (err = dev(&s->d_nseg, ng * n_cta)) || (err = dev(&s->d_nbar, M)) || (err = dev(&s->d_bar, 2 * M)) ||
-      (err = dev(&s->d_drift, 3 * M)) || (err = dev(&s->d_abort, 1)) ||
-      (err = dev(&s->d_spill, 3 * (size_t)e->total_nodes)) ||
-      (err = dev(&s->d_slot, (size_t)n_cta * 4 * kOverlap * nx_max)))
+      (err = dev(&s->d_nseg, ng * n_cta)) || (err = dev(&s->d_nbar, M)) || (err = dev(&s->d_bar, 3 * M)) ||
+      (err = dev(&s->d_drift, M)) || (err = dev(&s->d_abort, 1)) || (err = dev(&s->d_tag, 1)) ||
+      (err = dev(&s->d_spill, 3 * (size_t)e->total_nodes)) || (err = dev(&s->d_slot, slots)))
     return err;
+  const uint32_t first_tag = 1;  // the slots start at 0
+
   if ((err = cudaMemcpy(s->d_groups, groups.data(), sizeof(SpanGroup) * ng, cudaMemcpyHostToDevice)) ||
       (err = cudaMemcpy(s->d_rowoff, rowoff.data(), sizeof(int32_t) * (M + 1), cudaMemcpyHostToDevice)) ||
       (err = cudaMemcpy(s->d_fallback, table.data(), sizeof(int32_t) * table.size(), cudaMemcpyHostToDevice)) ||
-      (err = cudaMemset(s->d_drift, 0, sizeof(int32_t) * 3 * M)) ||
+      (err = cudaMemcpy(s->d_tag, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice)) ||
+      (err = cudaMemset(s->d_slot, 0, sizeof(uint4) * slots)) ||
+      (err = cudaMemset(s->d_drift, 0, sizeof(int32_t) * M)) ||
       (err = cudaMemset(s->d_spill, 0, sizeof(float4) * 3 * (size_t)std::max<int64_t>(e->total_nodes, 1))))
     return err;
   return cudaSuccess;
@@ -986,6 +1046,7 @@ cudaError_t jf_span_launch(jf_engine* e, int K) {
   a.bar = s->d_bar;
   a.drift = s->d_drift;
   a.abort = s->d_abort;
+  a.tag = s->d_tag;
   a.spill = s->d_spill;
   a.slot = s->d_slot;
   a.grid = e->d_grid;
@@ -994,13 +1055,13 @@ cudaError_t jf_span_launch(jf_engine* e, int K) {
   a.t_dev = e->d_time;
   a.nodes = e->total_nodes;
   a.M = e->M;
-  a.nx_max = s->nx_max;
   a.stride = e->max_cells + 2;
   a.K = K;
   a.dt = (float)e->dt;
   for (size_t g = 0; g < s->groups.size(); ++g) {
     a.seg = s->d_seg + g * s->n_cta * kMaxSeg;
     a.nseg = s->d_nseg + g * s->n_cta;
+    a.tag_add = (uint32_t)(g * K);  // the groups share the slots
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(s->groups[g].n_cta, 1, 1);
     cfg.blockDim = dim3(s->threads, 1, 1);
@@ -1017,3 +1078,8 @@ cudaError_t jf_span_launch(jf_engine* e, int K) {
   }
   return cudaSuccess;
 }
+
+// Device counter of the substeps run so far, which tags their words, and what a
+// chunk of K substeps adds to it after its last launch.
+uint32_t* jf_span_tag(const jf_engine* e) { return e->span->d_tag; }
+uint32_t jf_span_tag_step(const jf_engine* e, int K) { return (uint32_t)(e->span->groups.size() * K); }
