@@ -180,10 +180,45 @@ __device__ __forceinline__ R block_pressure(const GradArgs<R>& a, int m) {
 // bit for bit.
 constexpr int kTileNodes = 1024;
 
+// The tile's sums.  A 64-bit shared-memory add is a compare-and-swap loop that
+// the lattice's neighbours, which share nodes, keep repeating; a 32-bit one is a
+// single instruction.  So the FP32 build splits a contribution v 2^44, rounded
+// to an integer, into hi 2^22 + lo with |lo| <= 2^21: hi is v 2^22 rounded, and
+// the rest of v is exact, so that rounding it rounds the whole.  Both halves
+// come from adding 1.5 2^23, which leaves the integer in the low bits, without
+// the slow 64-bit conversion.  32-bit sums of either hold a block's particles.
+// 8 tanks of 80,000 slots: forward 50.3 -> 37.9 us per substep, with the
+// backward 143 -> 121.
+template <class R> struct Tile;
+template <> struct Tile<float> {
+  int hi[3 * kTileNodes], lo[3 * kTileNodes];
+  __device__ __forceinline__ void clear(int e) { hi[e] = lo[e] = 0; }
+  static constexpr float kMax = 1.0f;  // contributions the split holds, |v| below
+  __device__ __forceinline__ void add(int e, float v) {
+    constexpr float kMagic = 12582912.0f;  // 1.5 2^23
+    const float t = __fadd_rn(__fmul_rn(v, 4194304.0f), kMagic);
+    const float h = __fsub_rn(t, kMagic);
+    const float r = __fmul_rn(__fmaf_rn(h, -2.3841858e-07f, v), kFix);  // (v - hi 2^-22) 2^44, exact
+    atomicAdd(hi + e, __float_as_int(t) - 0x4b400000);
+    atomicAdd(lo + e, __float_as_int(__fadd_rn(r, kMagic)) - 0x4b400000);
+  }
+  __device__ __forceinline__ unsigned long long get(int e) const {
+    return (unsigned long long)((long long)hi[e] * (1ll << 22) + (long long)lo[e]);
+  }
+};
+template <> struct Tile<double> {
+  double acc[3 * kTileNodes];
+  __device__ __forceinline__ void clear(int e) { acc[e] = 0.0; }
+  static constexpr double kMax = (double)kFixMax;
+  __device__ __forceinline__ void add(int e, double v) { atomicAdd(acc + e, v); }
+  __device__ __forceinline__ double get(int e) const { return acc[e]; }
+};
+static_assert(kT <= 512, "a node takes one contribution of each particle of a block");
+
 template <class R>
 __global__ void __launch_bounds__(kT) gf_p2g(GradArgs<R> a) {
   using Acc = typename GT<R>::Acc;
-  __shared__ Acc s_acc[3 * kTileNodes];
+  __shared__ Tile<R> s_acc;
   __shared__ int s_box[4];  // stencil bases: min x, min y, max x, max y
   const int m = blockIdx.y;
   const R pressure = block_pressure(a, m);
@@ -226,44 +261,50 @@ __global__ void __launch_bounds__(kT) gf_p2g(GradArgs<R> a) {
   const int W = s_box[2] - x0 + 3, H = s_box[3] - y0 + 3;
   if (s_box[2] < 0) return;  // no particle of the block scatters (uniform)
   Acc* fix = a.fix + 3 * I.g_off;
-  if (W * H > kTileNodes) {  // uniform: the direct path
-    if (!valid) return;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const auto c = jf_node_contrib_strict(I, st, sc, i, j);
-        const int64_t n = 3 * ((int64_t)(st.by + j) * I.nx + st.bx + i);
-        add_fixed(fix + n + 0, c.x, a.err + m);
-        add_fixed(fix + n + 1, c.y, a.err + m);
-        add_fixed(fix + n + 2, c.z, a.err + m);
-      }
+  auto scatter_direct = [&]() {
+    for (int k = 0; k < 9; ++k) {
+      const int i = k / 3, j = k - 3 * i;
+      const auto c = jf_node_contrib_strict(I, st, sc, i, j);
+      const int64_t n = 3 * ((int64_t)(st.by + j) * I.nx + st.bx + i);
+      add_fixed(fix + n + 0, c.x, a.err + m);
+      add_fixed(fix + n + 1, c.y, a.err + m);
+      add_fixed(fix + n + 2, c.z, a.err + m);
     }
+  };
+  if (W * H > kTileNodes) {  // uniform: the direct path
+    if (valid) scatter_direct();
     return;
   }
   const int entries = 3 * W * H;
-  for (int e = threadIdx.x; e < entries; e += blockDim.x) s_acc[e] = Acc(0);
+  for (int e = threadIdx.x; e < entries; e += blockDim.x) s_acc.clear(e);
   __syncthreads();
-  if (valid) {
+  // a bound on every contribution of the particle: weights are below 1 and node
+  // offsets within 1.5 dx
+  const R bound = fabs(sc.mv0) + fabs(sc.mv1) + fabs(sc.mass) +
+                  R(2) * I.dx * (fabs(sc.af00) + fabs(sc.af01) + fabs(sc.af10) + fabs(sc.af11));
+  if (valid && bound < Tile<R>::kMax) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         const auto c = jf_node_contrib_strict(I, st, sc, i, j);
-        Acc* t = s_acc + 3 * ((st.by + j - y0) * W + (st.bx + i - x0));
-        atomicAdd(t + 0, to_fixed(c.x, a.err + m));
-        atomicAdd(t + 1, to_fixed(c.y, a.err + m));
-        atomicAdd(t + 2, to_fixed(c.z, a.err + m));
+        const int t = 3 * ((st.by + j - y0) * W + (st.bx + i - x0));
+        s_acc.add(t + 0, c.x);
+        s_acc.add(t + 1, c.y);
+        s_acc.add(t + 2, c.z);
       }
     }
+  } else if (valid) {  // rare: straight to the grid, or flagged
+    scatter_direct();
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < entries; e += blockDim.x) {
-    const Acc v = s_acc[e];
-    if (v == Acc(0)) continue;
-    const int node = e / 3, comp = e - 3 * node;
-    const int ty = node / W, tx = node - ty * W;
-    atomicAdd(fix + 3 * ((int64_t)(y0 + ty) * I.nx + x0 + tx) + comp, v);
+  // a warp takes 32 consecutive entries of one tile row, consecutive in the grid too
+  const int row_n = 3 * W, chunks = (row_n + 31) >> 5;
+  for (int q = threadIdx.x >> 5; q < H * chunks; q += kT >> 5) {
+    const int ty = q / chunks, c = ((q - ty * chunks) << 5) + (threadIdx.x & 31);
+    if (c >= row_n) continue;
+    const Acc v = s_acc.get(ty * row_n + c);
+    if (v != Acc(0)) atomicAdd(fix + 3 * ((int64_t)(y0 + ty) * I.nx + x0) + c, v);
   }
 }
 
