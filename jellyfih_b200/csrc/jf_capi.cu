@@ -24,6 +24,7 @@ thread_local std::string g_create_err;
 constexpr int kHaloRows = 4;  // batched window rows beyond the band (1 below, 3 above)
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 1024;  // the chunk kernel's static shared variables, rounded up
+constexpr size_t kTankStageMax = (size_t)64 << 20;  // a larger tank fill gives its memory back at the next
 constexpr size_t kFramePiece = (size_t)1 << 22;  // pixels a frame read packs at a time: bounds its staging
 constexpr size_t kBandSlackSmem = 128 * 1024;  // window size up to which bands get spare rows
 
@@ -99,7 +100,7 @@ int upload_params(jf_engine* e) {
 // (e->n_live), so that the longest run first when the clusters do not all
 // fit at once: re-sorts the order and queues its upload.
 int upload_order(jf_engine* e) {
-  if (!e->d_order) return JF_OK;
+  if (!e->d_order || e->span) return JF_OK;  // spans balance by the rows' cost
   for (int q = 0; q < e->M; ++q) e->h_order[q] = q;
   std::stable_sort(e->h_order.begin(), e->h_order.end(),
                    [&](int32_t a, int32_t b) { return e->n_live[a] > e->n_live[b]; });
@@ -125,6 +126,19 @@ int need_slot_stage(jf_engine* e, size_t floats) {
   e->slot_stage_floats = 0;
   JF_CK(alloc(&e->d_slot_stage, floats), "cudaMalloc slot staging");
   e->slot_stage_floats = floats;
+  return JF_OK;
+}
+
+// The tank fill's working memory: at least `bytes`, kept with the engine, up to
+// kTankStageMax between calls.
+int need_tank_stage(jf_engine* e, size_t bytes) {
+  if (e->tank_stage_bytes >= bytes && (e->tank_stage_bytes <= kTankStageMax || bytes > kTankStageMax)) return JF_OK;
+  JF_CK(cudaStreamSynchronize(e->stream), "tank staging sync");
+  cudaFree(e->d_tank_stage);
+  e->d_tank_stage = nullptr;
+  e->tank_stage_bytes = 0;
+  JF_CK(cudaMalloc((void**)&e->d_tank_stage, std::max<size_t>(bytes, 16)), "cudaMalloc tank staging");
+  e->tank_stage_bytes = bytes;
   return JF_OK;
 }
 
@@ -453,7 +467,7 @@ int jf_destroy(jf_engine* e) {
   cudaFree(e->d_ep_stats); cudaFree(e->d_grid); cudaFree(e->d_stats); cudaFree(e->d_err);
   cudaFree(e->d_stage); cudaFree(e->d_stage_i); cudaFree(e->d_path);
   cudaFree(e->d_fit); cudaFree(e->d_fit_f); cudaFree(e->d_fit_i); cudaFree(e->d_time);
-  cudaFree(e->d_frame); cudaFree(e->d_vort); cudaFree(e->d_hue); cudaFree(e->d_slot_stage);
+  cudaFree(e->d_frame); cudaFree(e->d_vort); cudaFree(e->d_hue); cudaFree(e->d_slot_stage); cudaFree(e->d_tank_stage);
   if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
   for (auto& pr : e->step_events) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
   for (auto& pr : e->sort_events) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
@@ -555,19 +569,18 @@ int jf_load_robot(jf_engine* e, int32_t m, const double* robot_pos, const int32_
     }
   }
   // every robot particle excludes water, also those cut from the slots
-  double* d_robot = nullptr;
-  int32_t* d_scratch = nullptr;
   const int64_t scratch = jf_tank_scratch_ints(e, m, spacing_div);
   int32_t total = 0;
-  cudaError_t err = alloc(&d_robot, 2 * (size_t)std::max(n_robot, 1));
-  if (err == cudaSuccess) err = alloc(&d_scratch, (size_t)scratch);
-  if (err == cudaSuccess && n_robot > 0)
+  // the robot's positions, then the lattice's flags and counts
+  if ((rc = need_tank_stage(e, sizeof(double) * 2 * (size_t)n_robot + sizeof(int32_t) * (size_t)scratch))) return rc;
+  double* d_robot = e->d_tank_stage;
+  int32_t* d_scratch = reinterpret_cast<int32_t*>(d_robot + 2 * (size_t)n_robot);
+  cudaError_t err = cudaSuccess;
+  if (n_robot > 0)
     err = cudaMemcpyAsync(d_robot, robot_pos, sizeof(double) * 2 * n_robot, cudaMemcpyHostToDevice, e->stream);
   if (err == cudaSuccess)
     err = jf_tank_water_launch(e, m, d_robot, n_robot, bbox, water_margin, spacing_div, d_scratch, scratch, &total);
   if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
-  cudaFree(d_robot);
-  cudaFree(d_scratch);
   if (err != cudaSuccess) return cuda_fail(e, err, "tank water fill");
   const int32_t n_water = std::max(0, std::min(total, I.n_slots - n_robot));
   JF_CK(jf_load_launch(e, m, nr + n_water), "load kernel");

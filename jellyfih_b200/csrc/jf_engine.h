@@ -83,6 +83,8 @@ struct jf_engine {
   int32_t* d_stage_i = nullptr;    // staging for ints (max_slots * 2)
   float* d_slot_stage = nullptr;   // packed frames; plain path: slot-order reads and writes
   size_t slot_stage_floats = 0;
+  double* d_tank_stage = nullptr;  // tank fill: robot positions, lattice flags and counts
+  size_t tank_stage_bytes = 0;
   unsigned long long* d_path = nullptr;  // batched path counters (see jf_path_counts)
   double* d_fit = nullptr;         // fitness staging: M x 5 rows + M scores
   double* d_fit_f = nullptr;       // fitness staging: M contraction genes

@@ -16,7 +16,6 @@
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kRobotTile = 1024;  // robot positions per shared-memory tile (16 KB)
 
 struct Lattice {
   double x0, dx;  // x_i = x0 + i * dx
@@ -29,50 +28,40 @@ __device__ __forceinline__ double2 candidate(const Lattice& L, int64_t c) {
   return make_double2(__dadd_rn(L.x0, __dmul_rn((double)i, L.dx)), __dadd_rn(L.y0, __dmul_rn((double)j, L.dy)));
 }
 
-// keep[c] = 1 when candidate c is farther than `margin` from every robot
-// particle; per-block keep counts into block_count.
-__global__ void __launch_bounds__(kThreads) water_keep_kernel(Lattice L, const double2* __restrict__ robot,
-                                                             int n_robot, double4 bbox, double margin,
-                                                             int32_t* __restrict__ keep,
-                                                             int32_t* __restrict__ block_count) {
-  __shared__ double2 s_r[kRobotTile];
-  __shared__ int s_count[kThreads / 32];
-  const int64_t n = (int64_t)L.nx * L.ny;
+// drop[c] = 1 for the candidates within `margin` of a robot particle: a warp per
+// robot particle tests the few lattice points of the margin's box around it.
+// (Every candidate near the robot testing every robot particle was 2,000 pairs
+// in a row, 209 us for an 80,000-slot tank; this takes 4.)  The box is a point
+// wider than its rounding either way; candidates outside `bbox`, the robot's
+// box grown by the margin, keep.
+__global__ void __launch_bounds__(kThreads) robot_margin_kernel(Lattice L, const double2* __restrict__ robot,
+                                                               int n_robot, double4 bbox, double margin,
+                                                               uint8_t* __restrict__ drop) {
+  const int r = (int)((blockIdx.x * (int64_t)kThreads + threadIdx.x) >> 5);
+  if (r >= n_robot) return;
+  const double2 q = robot[r];
+  // a NaN position gives an empty box: it is near nothing
+  auto lo = [](double v, int n) { return (int)fmin(fmax(floor(v) - 1.0, 0.0), (double)n); };
+  auto hi = [](double v, int n) { return (int)fmin(fmax(ceil(v) + 1.0, -1.0), (double)(n - 1)); };
+  const int i0 = lo((q.x - margin - L.x0) / L.dx, L.nx), i1 = hi((q.x + margin - L.x0) / L.dx, L.nx);
+  const int j0 = lo((q.y - margin - L.y0) / L.dy, L.ny), j1 = hi((q.y + margin - L.y0) / L.dy, L.ny);
+  const int w = i1 - i0 + 1;
+  const int64_t n = w > 0 && j1 >= j0 ? (int64_t)w * (j1 - j0 + 1) : 0;
+  for (int64_t k = threadIdx.x & 31; k < n; k += 32) {
+    const int64_t c = (j0 + k / w) * L.nx + i0 + k % w;
+    const double2 p = candidate(L, c);
+    if (!(p.x >= bbox.x && p.x <= bbox.z && p.y >= bbox.y && p.y <= bbox.w)) continue;
+    const double ex = __dsub_rn(p.x, q.x), ey = __dsub_rn(p.y, q.y);
+    if (sqrt(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey))) <= margin) drop[c] = 1;
+  }
+}
+
+// Kept candidates per block.
+__global__ void __launch_bounds__(kThreads) water_count_kernel(int64_t n, const uint8_t* __restrict__ drop,
+                                                              int32_t* __restrict__ block_count) {
   const int64_t c = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  const bool valid = c < n;
-  const double2 p = valid ? candidate(L, c) : make_double2(0.0, 0.0);
-  // the robot's bounding box grown by the margin: candidates outside it keep
-  bool near = valid && p.x >= bbox.x && p.x <= bbox.z && p.y >= bbox.y && p.y <= bbox.w;
-  bool drop = false;
-  // the block scans the robot in tiles while any of its candidates needs it
-  if (__syncthreads_or(near)) {
-    for (int t0 = 0; t0 < n_robot; t0 += kRobotTile) {
-      const int tn = min(kRobotTile, n_robot - t0);
-      __syncthreads();
-      for (int k = threadIdx.x; k < tn; k += kThreads) s_r[k] = robot[t0 + k];
-      __syncthreads();
-      if (near && !drop) {
-        for (int k = 0; k < tn; ++k) {
-          const double ex = __dsub_rn(p.x, s_r[k].x), ey = __dsub_rn(p.y, s_r[k].y);
-          const double d2 = __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey));
-          if (sqrt(d2) <= margin) {
-            drop = true;
-            break;
-          }
-        }
-      }
-    }
-  }
-  const int kf = (valid && !drop) ? 1 : 0;
-  if (valid) keep[c] = kf;
-  const int wsum = __reduce_add_sync(0xffffffffu, kf);
-  if ((threadIdx.x & 31) == 0) s_count[threadIdx.x >> 5] = wsum;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int w = 0; w < kThreads / 32; ++w) s += s_count[w];
-    block_count[blockIdx.x] = s;
-  }
+  const int kept = __syncthreads_count(c < n && !drop[c]);
+  if (threadIdx.x == 0) block_count[blockIdx.x] = kept;
 }
 
 // Exclusive scan of the per-block counts (one block; blocks <= a few
@@ -115,14 +104,14 @@ __global__ void __launch_bounds__(1024) block_scan_kernel(int32_t* __restrict__ 
 
 // Kept candidate c goes to slot n_robot + (its rank among kept candidates),
 // if that is below n_slots: staging position (f32), material 0, fibre (0, 1).
-__global__ void __launch_bounds__(kThreads) water_place_kernel(Lattice L, const int32_t* __restrict__ keep,
+__global__ void __launch_bounds__(kThreads) water_place_kernel(Lattice L, const uint8_t* __restrict__ drop,
                                                               const int32_t* __restrict__ block_base,
                                                               int n_robot, int n_slots, float* __restrict__ pos,
                                                               float* __restrict__ fib, int32_t* __restrict__ mat) {
   __shared__ int s_warp[kThreads / 32];
   const int64_t n = (int64_t)L.nx * L.ny;
   const int64_t c = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  const int kf = c < n ? keep[c] : 0;
+  const int kf = c < n && !drop[c];
   const unsigned ballot = __ballot_sync(0xffffffffu, kf);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) s_warp[warp] = __popc(ballot);
@@ -163,22 +152,28 @@ cudaError_t jf_tank_water_launch(jf_engine* e, int m, const double* d_robot, int
   np_arange(margin, I.domain_h - margin, spacing, L.y0, L.dy, L.ny);
   const int64_t n = (int64_t)L.nx * L.ny;
   const int n_blocks = (int)((n + kThreads - 1) / kThreads);
-  // scratch: keep flags [n], block counts [n_blocks], total [1]
-  if (n + n_blocks + 1 > scratch_ints) return cudaErrorInvalidValue;
-  int32_t* keep = d_scratch;
-  int32_t* counts = d_scratch + n;
+  // scratch: block counts [n_blocks], total [1], drop flags (bytes) [n]
+  if (n_blocks + 1 + (n + 3) / 4 > scratch_ints) return cudaErrorInvalidValue;
+  int32_t* counts = d_scratch;
   int32_t* total = counts + n_blocks;
+  uint8_t* drop = reinterpret_cast<uint8_t*>(total + 1);
   const double4 box = make_double4(bbox[0] - water_margin, bbox[1] - water_margin, bbox[2] + water_margin,
                                    bbox[3] + water_margin);
   if (n_blocks > 0) {
-    water_keep_kernel<<<n_blocks, kThreads, 0, e->stream>>>(L, reinterpret_cast<const double2*>(d_robot), n_robot,
-                                                            box, water_margin, keep, counts);
+    cudaError_t err = cudaMemsetAsync(drop, 0, (size_t)n, e->stream);
+    if (err != cudaSuccess) return err;
+    if (n_robot > 0) {
+      robot_margin_kernel<<<(int)(((int64_t)n_robot * 32 + kThreads - 1) / kThreads), kThreads, 0, e->stream>>>(
+          L, reinterpret_cast<const double2*>(d_robot), n_robot, box, water_margin, drop);
+      e->launches += 1;
+    }
+    water_count_kernel<<<n_blocks, kThreads, 0, e->stream>>>(n, drop, counts);
     block_scan_kernel<<<1, 1024, 0, e->stream>>>(counts, n_blocks, total);
     const int64_t S = e->max_slots;
-    water_place_kernel<<<n_blocks, kThreads, 0, e->stream>>>(L, keep, counts, n_robot, I.n_slots, e->d_stage,
+    water_place_kernel<<<n_blocks, kThreads, 0, e->stream>>>(L, drop, counts, n_robot, I.n_slots, e->d_stage,
                                                              e->d_stage + 2 * S, e->d_stage_i);
     e->launches += 3;
-    cudaError_t err = cudaMemcpyAsync(h_total, total, sizeof(int32_t), cudaMemcpyDeviceToHost, e->stream);
+    err = cudaMemcpyAsync(h_total, total, sizeof(int32_t), cudaMemcpyDeviceToHost, e->stream);
     if (err != cudaSuccess) return err;
   } else {
     *h_total = 0;
@@ -195,5 +190,5 @@ int64_t jf_tank_scratch_ints(const jf_engine* e, int m, double spacing_div) {
   np_arange(margin, 1.0 - margin, spacing, x0, dx, nx);
   np_arange(margin, I.domain_h - margin, spacing, x0, dx, ny);
   const int64_t n = (int64_t)nx * ny;
-  return n + (n + kThreads - 1) / kThreads + 1;
+  return (n + 3) / 4 + (n + kThreads - 1) / kThreads + 1;
 }
