@@ -107,7 +107,8 @@ struct GradArgs {
   const JfParams* params;
   typename GT<R>::Mats mats;
   GradState<R> s;              // the state the kernel reads (pre-step)
-  GradState<R> o;              // where it writes the post-step state (s itself in the forward)
+  GradState<R> o;              // where it writes the state that follows (s itself in the forward)
+  GradState<R> keep;           // gf_step: where the state before this P2G is kept (a checkpoint), if set
   const int32_t* mat;
   R* Jp;
   const float2* fiber;
@@ -171,13 +172,16 @@ __device__ __forceinline__ R block_pressure(const GradArgs<R>& a, int m) {
   return s_p;
 }
 
-// Deterministic P2G.  A block's particles (consecutive slots of one
-// instance) first add their contributions into a shared-memory tile covering
-// the block's stencil bounding box, when that box has at most kTileNodes
-// nodes, and the tile then goes to the grid with one atomic per touched node
-// and component; otherwise each contribution goes to the grid directly.  In
-// FP32 the contributions are integers, so every grouping gives the same sums
-// bit for bit.
+// G2P of the substep before (kG2p), then the deterministic P2G of this one
+// (kP2g): between two grids a particle is read and written once.  x, v and C
+// come from s and go to o; F, which only P2G changes, likewise.
+//
+// P2G: a block's particles (consecutive slots of one instance) first add their
+// contributions into a shared-memory tile covering the block's stencil bounding
+// box, when that box has at most kTileNodes nodes, and the tile then goes to
+// the grid with one atomic per touched node and component; otherwise each
+// contribution goes to the grid directly.  In FP32 the contributions are
+// integers, so every grouping gives the same sums bit for bit.
 constexpr int kTileNodes = 1024;
 
 // The tile's sums.  A 64-bit shared-memory add is a compare-and-swap loop that
@@ -215,36 +219,57 @@ template <> struct Tile<double> {
 };
 static_assert(kT <= 512, "a node takes one contribution of each particle of a block");
 
-template <class R>
-__global__ void __launch_bounds__(kT) gf_p2g(GradArgs<R> a) {
+template <class R, bool kG2p, bool kP2g>
+__global__ void __launch_bounds__(kT) gf_step(GradArgs<R> a) {
   using Acc = typename GT<R>::Acc;
   __shared__ Tile<R> s_acc;
   __shared__ int s_box[4];  // stencil bases: min x, min y, max x, max y
   const int m = blockIdx.y;
-  const R pressure = block_pressure(a, m);
+  const R pressure = kP2g ? block_pressure(a, m) : R(0);
   const auto I = a.inst[m];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t g = I.p_off + k;
-  const bool copy = a.o.F != a.s.F;
   bool valid = false;
   typename GT<R>::Stencil st;
   typename GT<R>::Scatter sc;
-  if (k < I.n_slots) {
-    const int mt = a.mat[g];
-    const V4<R> xv = mt >= 0 ? a.s.xv[g] : mk4(R(0), R(0), R(0), R(0));
-    if (mt >= 0 && jf_stencil_strict(I, mk2(xv.x, xv.y), st)) {
+  const int mt = k < I.n_slots ? a.mat[g] : -1;
+  if (mt >= 0) {
+    const V4<R> xv = a.s.xv[g];
+    V2<R> x = mk2(xv.x, xv.y), v = mk2(xv.z, xv.w);
+    V4<R> C;
+    if constexpr (kG2p) {
+      const V2<R>* u = a.u + I.g_off;
+      const int nx = I.nx;
+      if (jf_stencil_strict(I, x, st)) {
+        jf_g2p_apic_nodes(I, st, v, C, [&](int i, int j) { return u[(st.by + j) * nx + st.bx + i]; });
+      } else {
+        C = a.s.C[g];
+      }
+      jf_g2p_advect(I, x, v);
+      if (!(isfinite(x.x) && isfinite(x.y) && isfinite(v.x) && isfinite(v.y))) atomicOr(a.err + m, 1);
+      a.o.xv[g] = mk4(x.x, x.y, v.x, v.y);
+      a.o.C[g] = C;
+    } else {
+      C = a.s.C[g];
+    }
+    if constexpr (kP2g) {
       V4<R> F = a.s.F[g];
-      R jp = (mt == 2) ? a.Jp[g] : R(1);
-      const float2 fb = (mt == 3) ? a.fiber[g] : make_float2(0.0f, 1.0f);
-      jf_p2g_particle(I, a.mats, mt, mk2(xv.z, xv.w), a.s.C[g], F, jp, fb, pressure,
-                      (R)a.params[m].payload_density, sc);
-      a.o.F[g] = F;
-      if (mt == 2) a.Jp[g] = jp;
-      valid = true;
-    } else if (copy) {
-      a.o.F[g] = a.s.F[g];
+      if (a.keep.xv) {
+        a.keep.xv[g] = mk4(x.x, x.y, v.x, v.y);
+        a.keep.C[g] = C;
+        a.keep.F[g] = F;
+      }
+      valid = jf_stencil_strict(I, x, st);
+      if (valid) {
+        R jp = (mt == 2) ? a.Jp[g] : R(1);
+        const float2 fb = (mt == 3) ? a.fiber[g] : make_float2(0.0f, 1.0f);
+        jf_p2g_particle(I, a.mats, mt, v, C, F, jp, fb, pressure, (R)a.params[m].payload_density, sc);
+        if (mt == 2) a.Jp[g] = jp;
+      }
+      if (valid || a.o.F != a.s.F) a.o.F[g] = F;
     }
   }
+  if constexpr (!kP2g) return;
   if (threadIdx.x == 0) {
     s_box[0] = s_box[1] = 0x7fffffff;
     s_box[2] = s_box[3] = -1;
@@ -308,45 +333,19 @@ __global__ void __launch_bounds__(kT) gf_p2g(GradArgs<R> a) {
   }
 }
 
+// The grid from the sums, which are cleared for the next substep.
 template <class R>
 __global__ void gf_grid(GradArgs<R> a) {
   const int m = blockIdx.y;
   const auto I = a.inst[m];
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= I.nx * I.ny) return;
-  const typename GT<R>::Acc* q = a.fix + 3 * (I.g_off + n);
+  using Acc = typename GT<R>::Acc;
+  Acc* q = a.fix + 3 * (I.g_off + n);
   const R px = from_fixed(q[0]), py = from_fixed(q[1]), pm = from_fixed(q[2]);
+  q[0] = q[1] = q[2] = Acc(0);
   a.u[I.g_off + n] = jf_grid_node(I, n % I.nx, n / I.nx, px, py, pm);
   if (a.pmv) a.pmv[I.g_off + n] = mk4(px, py, pm, R(0));
-}
-
-template <class R>
-__global__ void gf_g2p(GradArgs<R> a) {
-  const int m = blockIdx.y;
-  const auto I = a.inst[m];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= I.n_slots) return;
-  const int64_t g = I.p_off + k;
-  if (a.mat[g] < 0) {
-    if (a.o.xv != a.s.xv) {
-      a.o.xv[g] = a.s.xv[g];
-      a.o.C[g] = a.s.C[g];
-    }
-    return;
-  }
-  const V4<R> xv = a.s.xv[g];
-  V2<R> x = mk2(xv.x, xv.y), v = mk2(xv.z, xv.w);
-  V4<R> C = a.s.C[g];
-  const V2<R>* u = a.u + I.g_off;
-  const int nx = I.nx;
-  typename GT<R>::Stencil st;
-  if (jf_stencil_strict(I, x, st)) {
-    jf_g2p_apic_nodes(I, st, v, C, [&](int i, int j) { return u[(st.by + j) * nx + st.bx + i]; });
-  }
-  jf_g2p_advect(I, x, v);
-  if (!(isfinite(x.x) && isfinite(x.y) && isfinite(v.x) && isfinite(v.y))) atomicOr(a.err + m, 1);
-  a.o.xv[g] = mk4(x.x, x.y, v.x, v.y);
-  a.o.C[g] = C;
 }
 
 template <class R>
@@ -362,6 +361,7 @@ struct AdjArgs {
   double* gparam;      // M x 3: d/d actuation, d/d contraction, d/d freq
   double* dLdp;        // M: d L / d pressure of this substep, per instance
   double* fac;         // M x 3: d pressure / d (actuation, contraction, freq) of this substep
+  int32_t* n_floor;    // water at the singular-value floor in this substep: cleared by ad_grid
 };
 
 template <class R>
@@ -465,7 +465,10 @@ template <class R>
 __global__ void ad_grid(AdjArgs<R> A) {
   const GradArgs<R>& a = A.f;
   const int m = blockIdx.y;
-  if (blockIdx.x == 0 && threadIdx.x == 0) pressure_factors(a.params[m], a.t, A.fac + 3 * m);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    pressure_factors(a.params[m], a.t, A.fac + 3 * m);
+    if (m == 0) *A.n_floor = 0;
+  }
   const auto I = a.inst[m];
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= I.nx * I.ny) return;
@@ -473,6 +476,7 @@ __global__ void ad_grid(AdjArgs<R> A) {
   const V4<R> q = a.pmv[node];
   const R px = q.x, py = q.y, pm = q.z;
   const V2<R> ub = A.ubar[node];
+  A.ubar[node] = mk2(R(0), R(0));  // for the next substep's ad_g2p
   if (!(pm > R(0))) {
     A.pmbar[node] = mk4(ub.x, ub.y, R(0), R(0));
     return;
@@ -939,6 +943,7 @@ GradArgs<R> grad_args(jf_engine* e, GradState<R> s, R t) {
   a.mats = mats_of<R>();
   a.s = s;
   a.o = s;
+  a.keep = GradState<R>{nullptr, nullptr, nullptr};
   a.mat = e->p.mat;
   a.Jp = work_Jp<R>(e);
   a.fiber = e->p.fiber;
@@ -966,30 +971,23 @@ cudaError_t copy_state(jf_engine* e, GradState<R> dst, GradState<R> src, cudaStr
   return cudaMemcpyAsync(dst.F, src.F, bytes, cudaMemcpyDeviceToDevice, st);
 }
 
-// one deterministic substep of every instance from state s at time t into
-// state o (s itself when o is not given); with u_keep / pmv_keep set, its grid
-// is written there for the adjoint
+// One launch pair of the deterministic forward: G2P of the substep before, when
+// `first` is false, and P2G of this one, then this substep's grid.
 template <class R>
-cudaError_t det_substep(jf_engine* e, GradState<R> s, R t, V2<R>* u_keep = nullptr, V4<R>* pmv_keep = nullptr,
-                        const GradState<R>* o = nullptr, cudaStream_t st = nullptr) {
-  if (!st) st = e->stream;
-  GradBuffers<R>& G = bufs<R>(e);
-  GradArgs<R> a = grad_args<R>(e, s, t);
-  if (o) a.o = *o;
-  if (u_keep) {
-    a.u = u_keep;
-    a.pmv = pmv_keep;
-  }
-  cudaError_t err = cudaMemsetAsync(G.fix, 0, sizeof(typename GT<R>::Acc) * 3 * (size_t)e->total_nodes, st);
-  if (err != cudaSuccess) return err;
+cudaError_t det_substep(jf_engine* e, const GradArgs<R>& a, const GradArgs<R>& grid, bool first, cudaStream_t st) {
   const dim3 gp((e->max_slots + kT - 1) / kT, e->M), gn((e->max_cells + kT - 1) / kT, e->M);
-  gf_p2g<R><<<gp, kT, 0, st>>>(a);
-  gf_grid<R><<<gn, kT, 0, st>>>(a);
-  gf_g2p<R><<<gp, kT, 0, st>>>(a);
-  e->launches += 3;
+  if (first) gf_step<R, false, true><<<gp, kT, 0, st>>>(a);
+  else gf_step<R, true, true><<<gp, kT, 0, st>>>(a);
+  gf_grid<R><<<gn, kT, 0, st>>>(grid);
+  e->launches += 2;
   return cudaGetLastError();
 }
 
+// The P2G sums cleared before a run of substeps (gf_grid leaves them so).
+template <class R>
+cudaError_t clear_sums(jf_engine* e, cudaStream_t st) {
+  return cudaMemsetAsync(bufs<R>(e).fix, 0, sizeof(typename GT<R>::Acc) * 3 * (size_t)e->total_nodes, st);
+}
 
 // Every buffer of a rollout of `steps` substeps with a checkpoint every K
 // (allocated before any graph capture: capture allows no allocation).
@@ -1137,14 +1135,17 @@ cudaError_t fwd_record(jf_engine* e) {
   if ((err = widen<R>(e))) return err;
   const GradState<R> work = work_state<R>(e);
   const std::vector<R> ts = substep_times<R>(e, G.t0, steps);
+  if ((err = clear_sums<R>(e, e->stream))) return err;
   for (int64_t s = 0; s < steps; ++s) {
-    if (s % K == 0) {
-      if ((err = copy_state<R>(e, state_at<R>(G.ck, slots, s / K), work)) != cudaSuccess) return err;
-    }
-    {
-      JfTimed timed(e, false);
-      if ((err = det_substep<R>(e, work, ts[(size_t)s])) != cudaSuccess) return err;
-    }
+    JfTimed timed(e, false);
+    GradArgs<R> a = grad_args<R>(e, work, ts[(size_t)s]);
+    if (s % K == 0) a.keep = state_at<R>(G.ck, slots, (size_t)(s / K));
+    if ((err = det_substep<R>(e, a, a, s == 0, e->stream)) != cudaSuccess) return err;
+  }
+  {
+    const dim3 gp((e->max_slots + kT - 1) / kT, e->M);
+    gf_step<R, true, false><<<gp, kT, 0, e->stream>>>(grad_args<R>(e, work, ts[(size_t)steps]));
+    e->launches += 1;
   }
   if ((err = copy_state<R>(e, state_at<R>(G.fin, slots, 0), work)) != cudaSuccess) return err;
   if ((err = cudaMemcpyAsync(G.fin_Jp, work_Jp<R>(e), sizeof(R) * slots, cudaMemcpyDeviceToDevice, e->stream)))
@@ -1217,6 +1218,7 @@ cudaError_t bwd_record(jf_engine* e) {
   cudaError_t err = cudaMemsetAsync(G.gparam, 0, sizeof(double) * 3 * e->M, e->stream);
   if (err != cudaSuccess) return err;
   if ((err = cudaMemsetAsync(G.dLdp, 0, sizeof(double) * (size_t)steps * e->M, e->stream))) return err;
+  if ((err = cudaMemsetAsync(G.ubar, 0, sizeof(V2<R>) * (size_t)e->total_nodes, e->stream))) return err;
   seed_kernel<R><<<gp, kT, 0, e->stream>>>(e->d_inst, e->p.mat, G.body_mode, G.inv_n, G.lxv, G.lC, G.lF, 1, R(1));
   e->launches += 1;
   const GradState<R> work = work_state<R>(e);
@@ -1226,8 +1228,7 @@ cudaError_t bwd_record(jf_engine* e) {
   const int floor_blocks = 16;         // water at the singular-value floor: rare
   auto seg_len = [&](int64_t seg) { return (int)((steps - seg * K) < K ? (steps - seg * K) : K); };
   // Recompute of segment `seg` into buffer set b on the recompute stream: its
-  // pre-step states (substep j reads state j and writes state j + 1; the last
-  // writes the working state, which nothing reads) and every substep's grid.
+  // pre-step states and every substep's grid.
   // It waits until the adjoint that last read buffer set b is done.  The
   // recompute needs only its checkpoint, so it runs while the main stream
   // runs the adjoint of the segment after it.
@@ -1237,12 +1238,21 @@ cudaError_t bwd_record(jf_engine* e) {
     if ((r = copy_state<R>(e, state_at<R>(G.seg[b], slots, 0), state_at<R>(G.ck, slots, (size_t)seg),
                            G.rstream)))
       return r;
+    if ((r = clear_sums<R>(e, G.rstream))) return r;
     const int n = seg_len(seg);
     for (int j = 0; j < n; ++j) {
-      const GradState<R> next = (j + 1 < n) ? state_at<R>(G.seg[b], slots, (size_t)j + 1) : work;
-      if ((r = det_substep<R>(e, state_at<R>(G.seg[b], slots, (size_t)j), ts[seg * K + j], G.useg[b] + nodes * j,
-                              G.pmseg[b] + nodes * j, &next, G.rstream)))
-        return r;
+      // x, v and C of state j from state j - 1 and its grid; F of state j + 1
+      // (after the last, of the working state, which nothing reads)
+      const GradState<R> here = state_at<R>(G.seg[b], slots, (size_t)j);
+      const GradState<R> from = j > 0 ? state_at<R>(G.seg[b], slots, (size_t)j - 1) : here;
+      const GradState<R> next = j + 1 < n ? state_at<R>(G.seg[b], slots, (size_t)j + 1) : work;
+      GradArgs<R> a = grad_args<R>(e, GradState<R>{from.xv, from.C, here.F}, ts[seg * K + j]);
+      a.o = GradState<R>{here.xv, here.C, next.F};
+      if (j > 0) a.u = G.useg[b] + nodes * (j - 1);
+      GradArgs<R> grid = a;
+      grid.u = G.useg[b] + nodes * j;
+      grid.pmv = G.pmseg[b] + nodes * j;
+      if ((r = det_substep<R>(e, a, grid, j == 0, G.rstream))) return r;
     }
     return cudaEventRecord(G.ready[b], G.rstream);
   };
@@ -1271,11 +1281,10 @@ cudaError_t bwd_record(jf_engine* e) {
       A.gparam = G.gparam;
       A.dLdp = G.dLdp + (size_t)(s0 + j) * e->M;
       A.fac = G.fac;
+      A.n_floor = G.counts + 1;
       // the substep's grid as the recompute left it
       A.f.u = G.useg[b] + nodes * j;
       A.f.pmv = G.pmseg[b] + nodes * j;
-      if ((err = cudaMemsetAsync(G.ubar, 0, sizeof(V2<R>) * nodes, e->stream))) return err;
-      if ((err = cudaMemsetAsync(G.counts + 1, 0, sizeof(int32_t), e->stream))) return err;
       ad_g2p<R><<<gp, kT, 0, e->stream>>>(A);
       ad_grid<R><<<gn, kT, 0, e->stream>>>(A);
       // P2G adjoint: the non-water particles on the second stream, beside the water
