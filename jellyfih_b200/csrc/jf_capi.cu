@@ -519,9 +519,11 @@ int jf_load_instance(jf_engine* e, int32_t m, const float* pos, const int32_t* m
           "stage material");
   }
   JF_CK(jf_load_launch(e, m, n), "load kernel");
-  int32_t live = 0;
-  for (int k = 0; k < n; ++k) live += material[k] >= 0 ? 1 : 0;
-  if ((rc = set_live_count(e, m, live))) return rc;
+  if (e->d_order && !e->span) {
+    int32_t live = 0;
+    for (int k = 0; k < n; ++k) live += material[k] >= 0 ? 1 : 0;
+    if ((rc = set_live_count(e, m, live))) return rc;
+  }
   JF_CK(cudaStreamSynchronize(e->stream), "load sync");
   e->sorted = false;
   return JF_OK;
@@ -793,7 +795,7 @@ int jf_run_episode(jf_engine* e, const float* pos, const int32_t* material, cons
   }
   JF_CK(jf_load_all_launch(e, d_pos, e->d_ep_mat, fiber ? d_fib : nullptr, d_glow), "episode load");
   e->sorted = false;
-  if (e->d_order) {
+  if (e->d_order && !e->span) {  // the clusters' order; spans balance by the rows' cost
     for (size_t m = 0; m < M; ++m) {
       const JfInst& I = e->inst[m];
       int32_t live = 0;

@@ -51,13 +51,21 @@ constexpr int kOverlap = 4;       // rows around a cut that both sides hold
 constexpr int kSpanThreads = 512;
 constexpr int kScanThreads = 1024;
 constexpr int kMoveThreads = 256;
-// The cell cap and the row costs follow the same model as the cluster path's
-// sort (jf_batched.cu): 128 per warp iteration, 6 per overflow particle, 40
-// for a row's grid update, 1.5 per non-water particle.
+// What a pass costs, in units of 1/128 of a warp's iteration over its 32 cells:
+// the cell cap minimises, and the spans balance, 128 for every iteration of a
+// segment's fullest cell up to the cap, kOverCost for a particle beyond it
+// (scattered with atomics of its own), and for the spans also kSegCost for a
+// segment's flush, kRowCost for a row's grid update and kSolidCostHalves / 2
+// for a non-water particle.  Swept on running batches, us per substep: overflow
+// 4 / 6 / 10 / 14 / 24 / 64: 48 uneven beside 16 tall 431 / 242 / 218 / 212 /
+// 216 / 217, 32 tanks of 80,000 slots 148 / 74.1 / 74.2 / 74.1 / 74.0 / 73.9;
+// segment 0 / 64 / 128 / 192: 32 tanks 76.2 / 74.4 / 74.1 / 74.0.
 constexpr int kCapCandidates = 16;
 constexpr int kNoCap = 1 << 30;
-constexpr int kRowCost = 40;
-constexpr int kSolidCostHalves = 3;
+constexpr int kOverCost = 14;
+constexpr int kSegCost = 128;
+constexpr int kRowCost = 80;
+constexpr int kSolidCostHalves = 5;
 constexpr unsigned kSpinLimit = 4000000;  // polls of about 0.7 us each: some seconds
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 3072;  // static shared variables of the kernel, rounded up
@@ -585,7 +593,7 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
   if (tid < 3) bar[tid * M + m] = 0ull;
   if (tid == 0 && m == 0) *abort = 0;
 
-  // lane k sums the cost of candidate k (0 = no cap), in quarter lane-iterations
+  // lane k sums the cost of candidate k (0 = no cap)
   int cost = 0;
   for (int sg = warp; sg < I.ny * segs; sg += kWarps) {
     const int row = sg / segs, x = ((sg - row * segs) << 5) + lane;
@@ -597,7 +605,7 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
       const int o = (int)__reduce_add_sync(full, (unsigned)max(0, n - k));
       if (lane == k) ov = o;
     }
-    cost += 128 * (lane == 0 ? mx : min(mx, lane)) + 6 * ov;
+    cost += 128 * (lane == 0 ? mx : min(mx, lane)) + kOverCost * ov;
   }
   if (lane < kCapCandidates) atomicAdd(&s_cost[lane], cost);
   __syncthreads();
@@ -617,7 +625,7 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
     const int mx = (int)__reduce_max_sync(full, (unsigned)n);
     const int ov = (int)__reduce_add_sync(full, (unsigned)max(0, n - cap));
     if (lane == 0 && mx) {
-      atomicAdd(&s_row_cost[row], 128 * min(mx, cap) + 6 * ov);
+      atomicAdd(&s_row_cost[row], kSegCost + 128 * min(mx, cap) + kOverCost * ov);
       if (ov) atomicAdd(&s_row_over[row], ov);
     }
   }
@@ -697,8 +705,16 @@ __global__ void __launch_bounds__(kScanThreads) span_cut_kernel(
     int32_t* __restrict__ nbar) {
   __shared__ unsigned long long s_sum[kScanThreads / 32];
   __shared__ int s_cut[kScanThreads + 1];
+  __shared__ int s_off[kScanThreads + 1];
   __shared__ int s_used;
   const SpanGroup g = groups[blockIdx.x];
+  // row starts of the group's instances, near at hand for the serial walk below
+  const int n_inst = g.m1 - g.m0;
+  const bool near = n_inst <= kScanThreads;
+  if (near)
+    for (int q = threadIdx.x; q <= n_inst; q += kScanThreads) s_off[q] = rowoff[g.m0 + q] - g.row0;
+  auto row_start = [&](int m) { return near ? s_off[m - g.m0] : rowoff[m] - g.row0; };
+  const int nx = inst[g.m0].nx;  // the same for every instance
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned full = 0xffffffffu;
   const int32_t* cost = rowcost + g.row0;
@@ -744,17 +760,16 @@ __global__ void __launch_bounds__(kScanThreads) span_cut_kernel(
     for (int q = 1; q <= g.n_cta && prev < g.rows; ++q) {
       int y = q < g.n_cta ? s_cut[q] : g.rows;
       // instance of the span's first row, its rows [b, e) in the group
-      int b = rowoff[m] - g.row0, e = rowoff[m + 1] - g.row0;
+      int b = row_start(m), e = row_start(m + 1);
       while (prev >= e) {
         ++m;
         b = e;
-        e = rowoff[m + 1] - g.row0;
+        e = row_start(m + 1);
       }
       if (y < prev + kMinRows) y = prev + kMinRows;
       // walk its bands while they fit
       int at = prev, mm = m, bb = b, ee = e, room = cap_nodes, left = kMaxSeg;
       for (;;) {
-        const int nx = inst[mm].nx;
         int stop = min(y, ee);
         // a cut leaves at least kMinRows rows on either side within an instance
         if (stop < ee && ee - stop < kMinRows) stop = ee;
@@ -773,7 +788,7 @@ __global__ void __launch_bounds__(kScanThreads) span_cut_kernel(
         if (at < ee || at >= y || at >= g.rows) break;
         ++mm;
         bb = ee;
-        ee = rowoff[mm + 1] - g.row0;
+        ee = row_start(mm + 1);
       }
       if (at <= prev) {
         ok = false;
@@ -797,11 +812,11 @@ __global__ void __launch_bounds__(kScanThreads) span_cut_kernel(
       int m = g.m0, top = g.m1;  // instance of row lo
       while (top - m > 1) {
         const int mid = (m + top) >> 1;
-        if (rowoff[mid] - g.row0 <= lo) m = mid;
+        if (row_start(mid) <= lo) m = mid;
         else top = mid;
       }
       for (int at = lo; at < hi; ++m) {
-        const int b = rowoff[m] - g.row0, e = rowoff[m + 1] - g.row0;
+        const int b = row_start(m), e = row_start(m + 1);
         const int stop = min(hi, e);
         seg[((int64_t)blockIdx.x * n_cta_max + q) * kMaxSeg + n] = make_int4(m, at - b, stop - b, 0);
         atomicAdd(nbar + m, 1);
