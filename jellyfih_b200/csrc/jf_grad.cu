@@ -116,7 +116,9 @@ struct GradArgs {
   V2<R>* u;                    // updated grid velocity
   V4<R>* pmv;                  // if set: (momentum x, momentum y, mass) per node, kept for the adjoint
   int32_t* err;                // per-instance non-finite flags
+  R* press;                    // activation pressure per instance: gf_grid's for the substep after
   R t;
+  R t_next;                    // gf_grid: time of the substep after
 };
 
 // Largest contribution the P2G sums take: |v| < 64 keeps v * 2^44 below
@@ -160,13 +162,18 @@ __device__ __forceinline__ double activation(double freq, double contraction, do
   return jf_activation64(freq, contraction, t);
 }
 
+// Activation pressure of instance m at time t.
+template <class R>
+__device__ __forceinline__ R pressure_at(const JfParams& P, R t) {
+  return (R)P.actuation * activation((R)P.freq, (R)P.contraction, t);
+}
+
 // per-block activation pressure of instance blockIdx.y at time a.t
 template <class R>
 __device__ __forceinline__ R block_pressure(const GradArgs<R>& a, int m) {
   __shared__ R s_p;
   if (threadIdx.x == 0) {
-    const JfParams P = a.params[m];
-    s_p = (R)P.actuation * activation((R)P.freq, (R)P.contraction, a.t);
+    s_p = pressure_at(a.params[m], a.t);
   }
   __syncthreads();
   return s_p;
@@ -225,7 +232,9 @@ __global__ void __launch_bounds__(kT) gf_step(GradArgs<R> a) {
   __shared__ Tile<R> s_acc;
   __shared__ int s_box[4];  // stencil bases: min x, min y, max x, max y
   const int m = blockIdx.y;
-  const R pressure = kP2g ? block_pressure(a, m) : R(0);
+  // The waveform's double-precision cosine is some thousand cycles that a block
+  // would wait for: after the first substep the grid kernel before has it ready.
+  const R pressure = !kP2g ? R(0) : (kG2p ? a.press[m] : block_pressure(a, m));
   const auto I = a.inst[m];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t g = I.p_off + k;
@@ -275,11 +284,18 @@ __global__ void __launch_bounds__(kT) gf_step(GradArgs<R> a) {
     s_box[2] = s_box[3] = -1;
   }
   __syncthreads();
-  if (valid) {
-    atomicMin(&s_box[0], st.bx);
-    atomicMin(&s_box[1], st.by);
-    atomicMax(&s_box[2], st.bx);
-    atomicMax(&s_box[3], st.by);
+  {
+    const unsigned full = 0xffffffffu;
+    const int x_lo = __reduce_min_sync(full, valid ? st.bx : 0x7fffffff);
+    const int y_lo = __reduce_min_sync(full, valid ? st.by : 0x7fffffff);
+    const int x_hi = __reduce_max_sync(full, valid ? st.bx : -1);
+    const int y_hi = __reduce_max_sync(full, valid ? st.by : -1);
+    if ((threadIdx.x & 31) == 0 && x_hi >= 0) {
+      atomicMin(&s_box[0], x_lo);
+      atomicMin(&s_box[1], y_lo);
+      atomicMax(&s_box[2], x_hi);
+      atomicMax(&s_box[3], y_hi);
+    }
   }
   __syncthreads();
   const int x0 = s_box[0], y0 = s_box[1];
@@ -339,6 +355,7 @@ __global__ void gf_grid(GradArgs<R> a) {
   const int m = blockIdx.y;
   const auto I = a.inst[m];
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.press[m] = pressure_at(a.params[m], a.t_next);
   if (n >= I.nx * I.ny) return;
   using Acc = typename GT<R>::Acc;
   Acc* q = a.fix + 3 * (I.g_off + n);
@@ -818,6 +835,7 @@ struct GradBuffers {
   double* gparam = nullptr;
   double* dLdp = nullptr;  // steps x M: d L / d pressure per substep and instance
   size_t dLdp_cap = 0;
+  R* press = nullptr;          // M: activation pressure of the next substep
   double* fac = nullptr;       // M x 3 pressure factors of the current substep
   int32_t* solid = nullptr;    // the rollout's non-water live particles
   int32_t* floor_list = nullptr;  // water at the singular-value floor, per substep
@@ -844,7 +862,7 @@ struct GradBuffers {
     if (rstream) cudaStreamDestroy(rstream);
     for (GradGraph* gg : {&fwd_graph, &bwd_graph, &step_graph})
       if (gg->exec) cudaGraphExecDestroy(gg->exec);
-    cudaFree(dLdp); cudaFree(fac); cudaFree(solid); cudaFree(floor_list); cudaFree(counts);
+    cudaFree(dLdp); cudaFree(fac); cudaFree(press); cudaFree(solid); cudaFree(floor_list); cudaFree(counts);
     cudaFree(inst_of);
     if (side) cudaStreamDestroy(side);
     if (fork) cudaEventDestroy(fork);
@@ -951,7 +969,9 @@ GradArgs<R> grad_args(jf_engine* e, GradState<R> s, R t) {
   a.u = G.u;
   a.pmv = nullptr;
   a.err = e->d_err;
+  a.press = G.press;
   a.t = t;
+  a.t_next = t;
   return a;
 }
 
@@ -1014,6 +1034,7 @@ cudaError_t grad_alloc(jf_engine* e, int64_t steps, int32_t K) {
     if ((err = alloc_n(&G.body_mode, e->M)) != cudaSuccess) return err;
     if ((err = alloc_n(&G.inv_n, e->M)) != cudaSuccess) return err;
     if ((err = alloc_n(&G.fac, 3 * (size_t)e->M)) != cudaSuccess) return err;
+    if ((err = alloc_n(&G.press, (size_t)e->M)) != cudaSuccess) return err;
     if ((err = alloc_n(&G.solid, slots)) != cudaSuccess) return err;
     if ((err = alloc_n(&G.floor_list, slots)) != cudaSuccess) return err;
     if ((err = alloc_n(&G.counts, 2)) != cudaSuccess) return err;
@@ -1139,6 +1160,7 @@ cudaError_t fwd_record(jf_engine* e) {
   for (int64_t s = 0; s < steps; ++s) {
     JfTimed timed(e, false);
     GradArgs<R> a = grad_args<R>(e, work, ts[(size_t)s]);
+    a.t_next = ts[(size_t)s + 1];
     if (s % K == 0) a.keep = state_at<R>(G.ck, slots, (size_t)(s / K));
     if ((err = det_substep<R>(e, a, a, s == 0, e->stream)) != cudaSuccess) return err;
   }
@@ -1249,6 +1271,7 @@ cudaError_t bwd_record(jf_engine* e) {
       GradArgs<R> a = grad_args<R>(e, GradState<R>{from.xv, from.C, here.F}, ts[seg * K + j]);
       a.o = GradState<R>{here.xv, here.C, next.F};
       if (j > 0) a.u = G.useg[b] + nodes * (j - 1);
+      a.t_next = ts[seg * K + j + 1];
       GradArgs<R> grid = a;
       grid.u = G.useg[b] + nodes * j;
       grid.pmv = G.pmseg[b] + nodes * j;
