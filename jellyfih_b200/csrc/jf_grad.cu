@@ -189,6 +189,10 @@ __device__ __forceinline__ R block_pressure(const GradArgs<R>& a, int m) {
 // the grid with one atomic per touched node and component; otherwise each
 // contribution goes to the grid directly.  In FP32 the contributions are
 // integers, so every grouping gives the same sums bit for bit.
+//
+// Bound by its issue slots (68 % busy at 1,300 instructions a warp, a quarter of
+// them the tile's sums): five blocks per SM, 40 warps, rather than the four its
+// registers would give (256 tanks of 20,000 slots: forward 235 -> 227 us).
 constexpr int kTileNodes = 1024;
 
 // The tile's sums.  A 64-bit shared-memory add is a compare-and-swap loop that
@@ -227,7 +231,7 @@ template <> struct Tile<double> {
 static_assert(kT <= 512, "a node takes one contribution of each particle of a block");
 
 template <class R, bool kG2p, bool kP2g>
-__global__ void __launch_bounds__(kT) gf_step(GradArgs<R> a) {
+__global__ void __launch_bounds__(kT, sizeof(R) == 4 ? 5 : 1) gf_step(GradArgs<R> a) {
   using Acc = typename GT<R>::Acc;
   __shared__ Tile<R> s_acc;
   __shared__ int s_box[4];  // stencil bases: min x, min y, max x, max y
