@@ -372,7 +372,6 @@ __global__ void gf_grid(GradArgs<R> a) {
 template <class R>
 struct AdjArgs {
   GradArgs<R> f;       // pre-step state of this substep (segment buffer) and its kept grid (u, pmv)
-  const V4<R>* xnext;  // (x, v) after this substep, as the forward left it
   V4<R>* lxv;          // adjoint (x, v): in = post-step, out = pre-step
   V4<R>* lC;
   V4<R>* lF;
@@ -392,8 +391,8 @@ __device__ __forceinline__ R wd(int k, R f) {  // d W_k / d f
 }
 
 template <class R>
-__device__ __forceinline__ R clamp_pass(R x, R lo, R hi) {
-  return (x > lo && x < hi) ? R(1) : R(0);
+__device__ __forceinline__ R clamp_pass(R xpp, R lo, R hi) {
+  return (xpp > lo && xpp < hi) ? R(1) : R(0);
 }
 
 __device__ __forceinline__ void atomic_add2(float2* p, float a, float b) { atomicAdd(p, make_float2(a, b)); }
@@ -402,9 +401,6 @@ __device__ __forceinline__ void atomic_add2(double2* p, double a, double b) {
   atomicAdd(&p->y, b);
 }
 
-// Adjoint of G2P.  Whether the wall clamp passed a gradient is read from the
-// position it left: strictly between the bounds it is the position before the
-// clamp (gathering the velocity again to form that took a third of the kernel).
 template <class R>
 __global__ void ad_g2p(AdjArgs<R> A) {
   const GradArgs<R>& a = A.f;
@@ -415,16 +411,23 @@ __global__ void ad_g2p(AdjArgs<R> A) {
   const int64_t g = I.p_off + k;
   if (a.mat[g] < 0) return;
   const V4<R> xv = a.s.xv[g];
-  const V2<R> x = mk2(xv.x, xv.y);
+  V2<R> x = mk2(xv.x, xv.y), v = mk2(xv.z, xv.w);
   const V4<R> lxv = A.lxv[g];
   const V4<R> Cb = A.lC[g];
   typename GT<R>::Stencil st;
   const bool inr = jf_stencil_strict(I, x, st);
   const V2<R>* u = a.u + I.g_off;
   const int nx = I.nx;
-  const V4<R> xn = A.xnext[g];
-  const R xd0 = lxv.x * clamp_pass(xn.x, R(0.001), R(0.999));
-  const R xd1 = lxv.y * clamp_pass(xn.y, R(0.001), I.y_hi);
+  V2<R> vn = v;
+  if (inr) {
+    V4<R> Cn;
+    jf_g2p_apic_nodes(I, st, vn, Cn, [&](int i, int j) { return u[(st.by + j) * nx + st.bx + i]; });
+  }
+  vn.y = vn.y - I.dtg;
+  const R xpp0 = radd(x.x, rmul(I.dt, vn.x));
+  const R xpp1 = radd(x.y, rmul(I.dt, vn.y));
+  const R xd0 = lxv.x * clamp_pass(xpp0, R(0.001), R(0.999));
+  const R xd1 = lxv.y * clamp_pass(xpp1, R(0.001), I.y_hi);
   const R vt0 = lxv.z + I.dt * xd0;
   const R vt1 = lxv.w + I.dt * xd1;
   if (!inr) {
@@ -1295,9 +1298,6 @@ cudaError_t bwd_record(jf_engine* e) {
       JfTimed timed(e, false);
       AdjArgs<R> A;
       A.f = grad_args<R>(e, state_at<R>(G.seg[b], slots, (size_t)j), ts[s0 + j]);
-      A.xnext = j + 1 < n ? state_at<R>(G.seg[b], slots, (size_t)j + 1).xv
-                : seg + 1 < n_seg ? state_at<R>(G.ck, slots, (size_t)seg + 1).xv
-                                  : state_at<R>(G.fin, slots, 0).xv;
       A.lxv = G.lxv;
       A.lC = G.lC;
       A.lF = G.lF;
