@@ -96,6 +96,7 @@ struct JfSpan {
   int32_t total_rows = 0;
   int32_t cap_nodes = 0;   // window nodes of a CTA
   size_t smem = 0;
+  void* pool = nullptr;    // holds every array below
   SpanGroup* d_groups = nullptr;
   int32_t* d_rowoff = nullptr;    // M + 1: first row of each instance
   int32_t* d_rowcost = nullptr;   // total_rows
@@ -904,19 +905,12 @@ bool fill_cuts(const jf_engine* e, const SpanGroup& g, const std::vector<int32_t
   return true;
 }
 
-template <class T>
-cudaError_t dev(T** p, size_t n) {
-  return cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(n, 1));
-}
-
 }  // namespace
 
 void jf_span_free(jf_engine* e) {
   JfSpan* s = e->span;
   if (!s) return;
-  cudaFree(s->d_groups); cudaFree(s->d_rowoff); cudaFree(s->d_rowcost); cudaFree(s->d_rowpre); cudaFree(s->d_ovrow);
-  cudaFree(s->d_ovcur); cudaFree(s->d_fallback); cudaFree(s->d_seg); cudaFree(s->d_nseg); cudaFree(s->d_nbar);
-  cudaFree(s->d_bar); cudaFree(s->d_drift); cudaFree(s->d_abort); cudaFree(s->d_tag); cudaFree(s->d_spill); cudaFree(s->d_slot);
+  cudaFree(s->pool);
   delete s;
   e->span = nullptr;
 }
@@ -1004,24 +998,42 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
   s->smem = smem;
   const size_t slots = (size_t)n_cta * 4 * kOverlap * nx_max * ((e->flags & JF_FLAG_AXISYM) ? 2 : 1);
   const size_t ng = groups.size(), rows = (size_t)s->total_rows, M = (size_t)e->M;
-  if ((err = dev(&s->d_groups, ng)) || (err = dev(&s->d_rowoff, M + 1)) || (err = dev(&s->d_rowcost, rows)) ||
-      (err = dev(&s->d_rowpre, rows)) || (err = dev(&s->d_ovrow, rows + M)) || (err = dev(&s->d_ovcur, rows)) ||
-      (err = dev(&s->d_fallback, table.size())) || (err = dev(&s->d_seg, ng * n_cta * kMaxSeg)) ||
-      (err = dev(&s->d_nseg, ng * n_cta)) || (err = dev(&s->d_nbar, M)) || (err = dev(&s->d_bar, 3 * M)) ||
-      (err = dev(&s->d_drift, M)) || (err = dev(&s->d_abort, 1)) || (err = dev(&s->d_tag, 1)) ||
-      (err = dev(&s->d_spill, 3 * (size_t)e->total_nodes)) || (err = dev(&s->d_slot, slots)))
-    return err;
+  // one allocation for all of it: engines are made anew by callers that change shapes
+  size_t bytes = 0;
+  std::vector<std::pair<void**, size_t>> parts;
+  auto part = [&](auto** p, size_t n) {
+    parts.emplace_back((void**)p, bytes);
+    bytes += (sizeof(**p) * std::max<size_t>(n, 1) + 255) / 256 * 256;
+  };
+  part(&s->d_spill, 3 * (size_t)e->total_nodes);  // the first three are cleared
+  part(&s->d_slot, slots);
+  part(&s->d_drift, M);
+  const size_t zero_end = bytes;
+  part(&s->d_groups, ng);
+  part(&s->d_rowoff, M + 1);
+  part(&s->d_fallback, table.size());
+  part(&s->d_tag, 1);
+  part(&s->d_rowcost, rows);
+  part(&s->d_rowpre, rows);
+  part(&s->d_ovrow, rows + M);
+  part(&s->d_ovcur, rows);
+  part(&s->d_seg, ng * n_cta * kMaxSeg);
+  part(&s->d_nseg, ng * n_cta);
+  part(&s->d_nbar, M);
+  part(&s->d_bar, 3 * M);
+  part(&s->d_abort, 1);
+  if ((err = cudaMalloc(&s->pool, bytes))) return err;
+  for (auto& p : parts) *p.first = (char*)s->pool + p.second;
   const uint32_t first_tag = 1;  // the slots start at 0
-
-  if ((err = cudaMemcpy(s->d_groups, groups.data(), sizeof(SpanGroup) * ng, cudaMemcpyHostToDevice)) ||
-      (err = cudaMemcpy(s->d_rowoff, rowoff.data(), sizeof(int32_t) * (M + 1), cudaMemcpyHostToDevice)) ||
-      (err = cudaMemcpy(s->d_fallback, table.data(), sizeof(int32_t) * table.size(), cudaMemcpyHostToDevice)) ||
-      (err = cudaMemcpy(s->d_tag, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice)) ||
-      (err = cudaMemset(s->d_slot, 0, sizeof(uint4) * slots)) ||
-      (err = cudaMemset(s->d_drift, 0, sizeof(int32_t) * M)) ||
-      (err = cudaMemset(s->d_spill, 0, sizeof(float4) * 3 * (size_t)std::max<int64_t>(e->total_nodes, 1))))
+  if ((err = cudaMemsetAsync(s->pool, 0, zero_end, e->stream)) ||
+      (err = cudaMemcpyAsync(s->d_groups, groups.data(), sizeof(SpanGroup) * ng, cudaMemcpyHostToDevice, e->stream)) ||
+      (err = cudaMemcpyAsync(s->d_rowoff, rowoff.data(), sizeof(int32_t) * (M + 1), cudaMemcpyHostToDevice,
+                             e->stream)) ||
+      (err = cudaMemcpyAsync(s->d_fallback, table.data(), sizeof(int32_t) * table.size(), cudaMemcpyHostToDevice,
+                             e->stream)) ||
+      (err = cudaMemcpyAsync(s->d_tag, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice, e->stream)))
     return err;
-  return cudaSuccess;
+  return cudaStreamSynchronize(e->stream);
 }
 
 // The part of a re-sort after the cell keys: bins, spans, and the particles
