@@ -13,7 +13,7 @@ Inputs are synthetic (no reference datasets exist for this path).
 ``e2e`` repeats the workload through the public API with host buffers: every
 step loads each instance from pinned host memory, runs the episode with
 ``run_headless`` and reads the (M, 5) result back.  ``roofline`` rates the
-dominant kernel (the batched chunk kernel) at 100 algorithmic bytes per live
+dominant kernel (the batched path's span kernel) at 100 algorithmic bytes per live
 particle-substep (x, v, C, F read and written, material read) against the
 measured HBM copy bandwidth.  ``cpu_baseline`` times the CPU oracle (a
 restatement of the reference's substep) on the host cores.  ``plain`` times
@@ -172,7 +172,7 @@ def peaks():
 
 
 def traffic_per_particle_step():
-    """DRAM bytes per live particle-substep of the chunk kernel from the
+    """DRAM bytes per live particle-substep of the chunk's kernel from the
     committed ncu measurement, and the measurement's record.  The figure is
     None when the kernel's sources changed since that measurement (the file
     records a hash of them); the record still names the figure and the sources
@@ -645,7 +645,6 @@ def run_ours(args):
                     block_threads=args.block)
     stream = torch.cuda.Stream()
     engine.set_stream(stream)
-    layout = engine.layout()
     load_all(engine, inputs)
     engine.time = 0.0
 
@@ -687,7 +686,7 @@ def run_ours(args):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": (tpps * live * chunk_substeps) if tpps else None,
-                "kernel": "chunk_kernel", "algorithmic_bytes_per_launch": bytes_per_launch,
+                "kernel": "span_kernel", "algorithmic_bytes_per_launch": bytes_per_launch,
                 "mean_launch_ms": mean_launch_s * 1e3, "launches": kt["step_launches"],
                 "step_kernel_share": kt["step_ms"] / ms if ms > 0 else None,
                 "scatter_paths": paths,
@@ -779,7 +778,7 @@ def run_ours(args):
                                        f"FP32, {S} substeps per step",
                            "instances_per_gpu": M, "slots": args.slots, "live_particles": int(live_total),
                            "substeps_per_step": S, "resort_interval": args.resort,
-                           "block_threads": layout["block_threads"], "cluster_size": layout["cluster_size"],
+                           "layout": "spans of grid rows, one CTA per SM", "block_threads": args.block or 512,
                            "l2": "inputs larger than L2: particle state plus sort buffers ~260 MB per GPU",
                            "path": "batched"},
                 "roofline": roofline, "clocks": clocks.summary(), "gpu_launches": gpu_launches,
