@@ -66,7 +66,7 @@ constexpr int kOverCost = 14;
 constexpr int kSegCost = 128;
 constexpr int kRowCost = 80;
 constexpr int kSolidCostHalves = 5;
-constexpr unsigned kSpinLimit = 4000000;  // polls of about 0.7 us each: some seconds
+constexpr unsigned kSpinLimit = 20000000;  // polls of about 0.7 us each: some 14 seconds
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 3072;  // static shared variables of the kernel, rounded up
 // Shared memory and L1 share an SM's 256 KB: larger windows slow the particle
@@ -76,7 +76,8 @@ constexpr size_t kStaticSmem = 3072;  // static shared variables of the kernel, 
 // Measured on 48 instances of 40K to 120K particles on 128^2 beside 16 of 128K
 // on 128x256 (us per substep; shares of 200, 109, 80 and 65 KB): 1 group 325,
 // 2: 293, 3: 273, 4: 287; at 5/4 of the share 302 and 282 for 2 and 3 (some
-// re-sorts fell back to spans of equal windows).
+// re-sorts fell back to spans of equal windows).  With the cost model below 2, 3
+// and 4 groups take 216, 220 and 232.
 constexpr size_t kSoftSmem = 96 * 1024;
 
 struct SpanGroup {
@@ -252,8 +253,9 @@ __device__ __forceinline__ bool receive(const uint4* p, uint32_t tag, int32_t* a
 // registers (up to 512 threads, the default).  What bounds the pass is the
 // latency and the issue rate of the particles' FP32 chains at 16 warps per SM,
 // not memory: the state of the batch lives in L2.  Measured (us per substep,
-// 80K-slot tanks on 128^2, one cluster per instance before): 32 instances 98 ->
-// 82, 16: 107 -> 46, 8: 63 -> 27, 1: 35 -> 21.
+// 80K-slot tanks on 128^2) against one cluster per instance with the particle
+// code of the day: 32 instances 92.6 -> 82.6, 16: 91 -> 46, 8: 63 -> 27, 1: 35 ->
+// 21; now 75.9, 41, 24.4 and 16.0.
 template <bool kTmem, bool kAxisym, bool kGlow>
 __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(const __grid_constant__ SpanArgs a) {
   extern __shared__ float4 smem4[];
