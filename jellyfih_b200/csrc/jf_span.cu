@@ -440,8 +440,9 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
           s_seg[lane].P.actuation * jf_activation(s_seg[lane].P.freq, s_seg[lane].P.contraction, t);
 
     // grid update of one node of band S from its sums; `publish`: into global
-    // memory too
-    const bool last = (s == a.K - 1);
+    // memory too, which only follows the meeting: until then another CTA of the
+    // instance may be in this pass, whose drifted particles gather the rows that
+    // the substep before published
     auto update_node = [&](const SpanSeg& S, int wr, int i, float mx, float my, float mm, float mh, bool publish) {
       const int j = S.lo - kHaloLo + wr;
       const float2 u = jf_grid_node(S.I, i, j, mx, my, mm, mh);
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
       const int n0 = S.in_lo() * nx, n1 = S.in_hi() * nx;
       for (int n = n0 + tid; n < n1; n += nth) {
         const int wr = n / nx, o = S.off + n;
-        update_node(S, wr, n - wr * nx, Ax[o], Ay[o], Am[o], kAxisym ? Ah[o] : 0.0f, last);
+        update_node(S, wr, n - wr * nx, Ax[o], Ay[o], Am[o], kAxisym ? Ah[o] : 0.0f, false);
       }
     }
 #pragma unroll
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
         Ay[o] = my;
         Am[o] = mm;
         if (kAxisym) Ah[o] = mh;
-        update_node(S, wr0 + r, i, mx, my, mm, mh, last && (side ? r == 0 : r > 0));
+        update_node(S, wr0 + r, i, mx, my, mm, mh, false);
       }
     }
     if (tid < nseg) {
@@ -518,6 +519,11 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
           update_node(S, wr, i, Ax[o] + e.x, Ay[o] + e.y, Am[o] + e.z, kAxisym ? Ah[o] + e.w : 0.0f,
                       wr >= kHaloLo && wr < kHaloLo + rows);
         }
+      } else if (s == a.K - 1) {  // the chunk's last grid, of the rows it owns
+        for (int n = kHaloLo * nx + tid; n < (kHaloLo + rows) * nx; n += nth) {
+          const float2 u = G[S.off + n];
+          a.grid[S.I.g_off + (int64_t)(S.lo - kHaloLo) * nx + n] = make_float4(u.x, u.y, Am[S.off + n], 0.0f);
+        }
       }
       // the spill of the substep before has been read by everyone: its rows are cleared by their owners
       if (s > 0 && s_drift[(s - 1) & 1][q]) {
@@ -541,8 +547,9 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
         __threadfence();
       }
     }
-    // clear sums for the next pass
-    for (int n = tid; n < (kAxisym ? 4 : 3) * WN; n += nth) Ax[n] = 0.0f;
+    // clear sums for the next pass (the last one adds none, and the last grid is still being published)
+    if (s < a.K - 1)
+      for (int n = tid; n < (kAxisym ? 4 : 3) * WN; n += nth) Ax[n] = 0.0f;
     __syncthreads();
     if (any_drift && s_tot[3]) break;
   }
