@@ -286,10 +286,26 @@ int jf_read_frame(jf_engine* e, float* rgb);
 /* vort_grid of instance m (mpm_sim.py:106): vort[nx][ny]. */
 int jf_read_vorticity(jf_engine* e, int32_t m, float* vort);
 
-/* Per-instance non-finite flags raised by the G2P update since the last
- * clear (out[n_instances]). */
+/* Per-instance error flags raised since the last clear (out[n_instances]), 0
+ * or a sum of JF_ERRFLAG_*. */
+#define JF_ERRFLAG_NONFINITE 1   /* the G2P update gave a NaN or Inf */
+#define JF_ERRFLAG_RANGE 2       /* differentiable rollout: a P2G contribution was not finite or
+                                    reached 64, and was left out of the sums */
+#define JF_ERRFLAG_ADJOINT 4     /* differentiable rollout: a particle's adjoint was not finite */
+#define JF_ERRFLAG_ABANDONED 256 /* batched path: a thread block waited too long for another
+                                    (jf_set_wait_limit), and this instance was left unfinished,
+                                    in that chunk of substeps or in one queued behind it.  Nothing
+                                    steps until the flags are cleared; load the instances that
+                                    have this flag again after that.  The calls that synchronise
+                                    return JF_ERR_CUDA while it is set */
 int jf_error_flags(jf_engine* e, int32_t* out);
 int jf_clear_error_flags(jf_engine* e);
+
+/* How many polls, of about 0.7 us each, a thread block of the batched path
+ * waits for its neighbours' rows before it gives up; 0 restores the default of
+ * 2e7, some 14 seconds.  For batches that run as spans (jf_config.cluster_size);
+ * without effect otherwise.  No counterpart in the reference. */
+int jf_set_wait_limit(jf_engine* e, uint32_t polls);
 
 /* Batched path counters since the last reset (out has 4 entries): out[0]
  * particle scatters accumulated in a lane's register block, out[1] scatters

@@ -23,6 +23,10 @@ JF_FLAG_GLOW = 1
 JF_FLAG_NO_GRAPHS = 2
 JF_FLAG_AXISYM = 4
 JF_FLAG_GRAD_FP64 = 8
+JF_ERRFLAG_NONFINITE = 1
+JF_ERRFLAG_RANGE = 2
+JF_ERRFLAG_ADJOINT = 4
+JF_ERRFLAG_ABANDONED = 256
 JF_VORT_RDBU = 0
 JF_VORT_HUESHIFT = 1
 JF_VORT_WHITE = 2
@@ -89,6 +93,7 @@ EXPORTS = {
     "jf_read_vorticity": (ctypes.c_int, [_E, ctypes.c_int32, _P]),
     "jf_error_flags": (ctypes.c_int, [_E, _P]),
     "jf_clear_error_flags": (ctypes.c_int, [_E]),
+    "jf_set_wait_limit": (ctypes.c_int, [_E, ctypes.c_uint32]),
     "jf_kernel_launches": (ctypes.c_int64, [_E]),
     "jf_substep_noalloc": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                           ctypes.c_float, ctypes.c_double, ctypes.c_float,

@@ -646,7 +646,8 @@ static int nonfinite_status(jf_engine* e, const std::vector<int32_t>& flags) {
   for (int m = 0; m < e->M; ++m) {
     if (flags[m] & kJfErrAbort)
       return fail(e, JF_ERR_CUDA, "the step of instance " + std::to_string(m) +
-                                      " gave up waiting for another thread block; its state is not to be used");
+                                      " was given up: a thread block waited too long for another; clear the error "
+                                      "flags and load the instances that have them again");
     if (!flags[m]) continue;
     if (n < 8) which += (n ? ", " : "") + std::to_string(m);
     ++n;
@@ -1042,6 +1043,21 @@ int jf_clear_error_flags(jf_engine* e) {
   int rc = set_device(e);
   if (rc) return rc;
   JF_CK(cudaMemsetAsync(e->d_err, 0, sizeof(int32_t) * e->M, e->stream), "clear flags");
+  if (e->span) JF_CK(jf_span_clear_abort(e), "clear given-up wait");
+  return JF_OK;
+}
+
+int jf_set_wait_limit(jf_engine* e, uint32_t polls) {
+  if (check_engine(e)) return JF_ERR_INVALID;
+  int rc = set_device(e);
+  if (rc) return rc;
+  if (!e->span) return JF_OK;
+  jf_span_set_wait_limit(e, polls);
+  if (e->graph_exec) {  // the limit is among the captured launches' arguments
+    JF_CK(cudaStreamSynchronize(e->stream), "wait limit sync");
+    cudaGraphExecDestroy(e->graph_exec);
+    e->graph_exec = nullptr;
+  }
   return JF_OK;
 }
 

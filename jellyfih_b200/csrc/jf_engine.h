@@ -28,8 +28,9 @@ struct JfParticles {
 
 struct JfGrad;
 struct JfSpan;
-// Error flag of an instance whose chunk gave up waiting for another CTA.
-constexpr int32_t kJfErrAbort = 256;
+// Error flag of an instance left unfinished because a CTA gave up waiting for
+// another: one of its own, one that shares a CTA with it, or one of an earlier launch.
+constexpr int32_t kJfErrAbort = JF_ERRFLAG_ABANDONED;
 // Grids up to this many rows get bands balanced by per-row cost at each
 // re-sort (taller grids keep equal bands).
 constexpr int kJfMaxBandRows = 1024;
@@ -78,7 +79,7 @@ struct jf_engine {
   int32_t* d_solid = nullptr;      // batched path: M x kJfMaxBandRows non-water particles per grid row
   float4* d_grid = nullptr;        // grid nodes (node = g_off + j * nx + i): (v0, v1, m, 0)
   double* d_stats = nullptr;       // M x 6 CoM sums (payload y, count, x; body y, count, x)
-  int32_t* d_err = nullptr;        // per-instance non-finite flags
+  int32_t* d_err = nullptr;        // per-instance error flags (JF_ERRFLAG_*)
   float* d_stage = nullptr;        // host <-> device staging (max_slots * 8 floats)
   int32_t* d_stage_i = nullptr;    // staging for ints (max_slots * 2)
   float* d_slot_stage = nullptr;   // packed frames; plain path: slot-order reads and writes
@@ -151,6 +152,8 @@ cudaError_t jf_span_setup(jf_engine* e, int threads);
 cudaError_t jf_span_sort(jf_engine* e);
 cudaError_t jf_span_launch(jf_engine* e, int K);
 void jf_span_free(jf_engine* e);
+void jf_span_set_wait_limit(jf_engine* e, uint32_t polls);
+cudaError_t jf_span_clear_abort(jf_engine* e);
 uint32_t* jf_span_tag(const jf_engine* e);
 uint32_t jf_span_tag_step(const jf_engine* e, int K);
 

@@ -30,9 +30,12 @@
 // particle can gather them in the next pass.  The result does not depend on
 // the re-sort interval.
 //
-// Every wait counts its polls and gives up after kSpinLimit: the CTA raises
-// the abort flag, which ends the waits of the others, frees its tensor memory
-// and returns, and the instance's error flag kErrAbort is set.
+// Every wait counts its polls and gives up after spin_limit of them: the CTA
+// raises the abort flag, which ends the waits of the others, sets kJfErrAbort on
+// the instances of its bands, frees its tensor memory and returns.  The abort
+// flag stays up until jf_clear_error_flags: what is queued behind the chunk
+// returns at once, so that the time of a run whose waits run out is bounded by
+// one of them, and sets the same error flag on the instances it leaves alone.
 #include <algorithm>
 #include <utility>
 #include <vector>
@@ -66,7 +69,7 @@ constexpr int kOverCost = 14;
 constexpr int kSegCost = 128;
 constexpr int kRowCost = 80;
 constexpr int kSolidCostHalves = 5;
-constexpr unsigned kSpinLimit = 20000000;  // polls of about 0.7 us each: some 14 seconds
+constexpr uint32_t kSpinLimit = 20000000;  // default: polls of about 0.7 us each, some 14 seconds
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 3072;  // static shared variables of the kernel, rounded up
 // Shared memory and L1 share an SM's 256 KB: larger windows slow the particle
@@ -110,9 +113,10 @@ struct JfSpan {
   int32_t* d_nbar = nullptr;      // M: CTAs that hold a band of the instance
   // 3 M: arrivals of even and of odd substeps (drift marks in the upper half), of drift meetings
   unsigned long long* d_bar = nullptr;
-  int32_t* d_drift = nullptr;     // M: bit s % 3: the spill grid of substep s is in use
+  int32_t* d_drift = nullptr;     // M: bit s % 3: the spill grid of substep s is in use; kDriftUnknown
   uint32_t* d_tag = nullptr;      // tag of the next chunk's first substep
-  int32_t* d_abort = nullptr;
+  int32_t* d_abort = nullptr;     // a wait gave up: nothing runs until it is cleared
+  uint32_t spin_limit = kSpinLimit;
   float4* d_spill = nullptr;      // 3 x total nodes
   // n_cta x 2 sides x 2 parities x kOverlap x nx_max nodes (twice that, the hoop
   // sums in the second half, in the axisymmetric variant)
@@ -145,6 +149,7 @@ struct SpanArgs {
   unsigned long long* bar;
   int32_t* drift;
   int32_t* abort;
+  uint32_t spin_limit;        // polls after which a wait gives up
   const uint32_t* tag;        // counter of the substeps run so far
   uint32_t tag_add;           // of the groups launched before this one in the chunk
   float4* spill;
@@ -200,30 +205,31 @@ struct SpanWindow : JfWindow {
 };
 
 constexpr unsigned long long kMark = 1ull << 40;  // a drift mark in an arrival count
+constexpr int kDriftUnknown = 8;  // beside the drift bits: a CTA gave up, any of the spill grids may be in use
 
 __device__ __forceinline__ void arrive(unsigned long long* p, unsigned long long n) {
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(n) : "memory");
 }
 
 // One poll of a wait; false when the wait gave up or another CTA did.
-__device__ __forceinline__ bool keep_polling(unsigned& n, int32_t* abort) {
-  if (++n >= kSpinLimit) {
-    atomicExch(abort, 1);
+__device__ __forceinline__ bool keep_polling(uint32_t& n, const SpanArgs& a) {
+  if (++n >= a.spin_limit) {
+    atomicExch(a.abort, 1);
     return false;
   }
-  return (n & 63u) != 0u || *(volatile int32_t*)abort == 0;
+  return (n & 63u) != 0u || *(volatile int32_t*)a.abort == 0;
 }
 
 // Waits until the arrivals at *p have reached `target` (they only grow within a
 // launch); *seen is the count with its marks.
-__device__ __forceinline__ bool wait_for(const unsigned long long* p, unsigned long long target, int32_t* abort,
+__device__ __forceinline__ bool wait_for(const unsigned long long* p, unsigned long long target, const SpanArgs& a,
                                          unsigned long long* seen) {
-  for (unsigned n = 0;;) {
+  for (uint32_t n = 0;;) {
     unsigned long long v;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     *seen = v;
     if ((v & (kMark - 1)) >= target) return true;
-    if (!keep_polling(n, abort)) return false;
+    if (!keep_polling(n, a)) return false;
   }
 }
 
@@ -235,8 +241,8 @@ __device__ __forceinline__ void send(uint4* p, float a, float b, float c, uint32
       "f"(a), "f"(b), "f"(c), "r"(tag)
       : "memory");
 }
-__device__ __forceinline__ bool receive(const uint4* p, uint32_t tag, int32_t* abort, float3* v) {
-  for (unsigned n = 0;;) {
+__device__ __forceinline__ bool receive(const uint4* p, uint32_t tag, const SpanArgs& a, float3* v) {
+  for (uint32_t n = 0;;) {
     uint32_t t;
     asm volatile(
         "{\n\t.reg .b128 w;\n\t.reg .b64 l, h;\n\tld.relaxed.gpu.global.b128 w, [%4];\n\tmov.b128 {l, h}, w;\n\t"
@@ -245,7 +251,7 @@ __device__ __forceinline__ bool receive(const uint4* p, uint32_t tag, int32_t* a
         : "l"(p)
         : "memory");
     if (t == tag) return true;
-    if (!keep_polling(n, abort)) return false;
+    if (!keep_polling(n, a)) return false;
   }
 }
 
@@ -300,7 +306,12 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
     s_drift[0][tid] = s_drift[1][tid] = 0;
   }
   if (tid < 4) s_path[tid] = 0u;
+  if (tid == 0) s_tot[3] = *(volatile int32_t*)a.abort;
   __syncthreads();
+  if (s_tot[3]) {
+    if (tid < nseg) atomicOr(a.err + s_seg[tid].m, kJfErrAbort);
+    return;
+  }
   float t = *a.t_dev;
   const uint32_t tag0 = *a.tag + a.tag_add;
   if (tid == 0) {
@@ -317,7 +328,6 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
     s_tot[0] = gen;
     s_tot[1] = gen + cell;
     s_tot[2] = off;
-    s_tot[3] = 0;
     s_next_task[0] = n_warps;
   }
   if (tid < nseg)
@@ -470,9 +480,8 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
         const int r = n / nx, i = n - r * nx;
         const int o = S.off + wr0 * nx + n;
         float3 b, h = make_float3(0.0f, 0.0f, 0.0f);
-        if (!receive(from + n, tag, a.abort, &b) || (kAxisym && !receive(from + slot_half + n, tag, a.abort, &h))) {
+        if (!receive(from + n, tag, a, &b) || (kAxisym && !receive(from + slot_half + n, tag, a, &h))) {
           s_tot[3] = 1;
-          atomicOr(a.err + S.m, kJfErrAbort);
           break;
         }
         // both sides' sums, kept for a spill
@@ -490,10 +499,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
       int drift = 0;
       if (S.n_bar > 1) {
         unsigned long long seen;
-        if (!wait_for(a.bar + (s & 1) * a.M + S.m, (unsigned long long)(s / 2 + 1) * S.n_bar, a.abort, &seen)) {
-          s_tot[3] = 1;
-          atomicOr(a.err + S.m, kJfErrAbort);
-        }
+        if (!wait_for(a.bar + (s & 1) * a.M + S.m, (unsigned long long)(s / 2 + 1) * S.n_bar, a, &seen)) s_tot[3] = 1;
         const unsigned marks = (unsigned)(seen >> 40);
         drift = marks != S.marks[s & 1];
         S.marks[s & 1] = marks;
@@ -540,10 +546,7 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
         __threadfence();
         arrive(a.bar + 2 * a.M + S.m, 1);
         unsigned long long seen;
-        if (!wait_for(a.bar + 2 * a.M + S.m, (unsigned long long)S.n_meet2 * S.n_bar, a.abort, &seen)) {
-          s_tot[3] = 1;
-          atomicOr(a.err + S.m, kJfErrAbort);
-        }
+        if (!wait_for(a.bar + 2 * a.M + S.m, (unsigned long long)S.n_meet2 * S.n_bar, a, &seen)) s_tot[3] = 1;
         __threadfence();
       }
     }
@@ -552,6 +555,11 @@ __global__ void __launch_bounds__(kTmem ? kTmemThreads : 512, 1) span_kernel(con
       for (int n = tid; n < (kAxisym ? 4 : 3) * WN; n += nth) Ax[n] = 0.0f;
     __syncthreads();
     if (any_drift && s_tot[3]) break;
+  }
+  // all that the CTA's bands belong to is left in the middle of the chunk
+  if (s_tot[3] && tid < nseg) {
+    atomicOr(a.err + s_seg[tid].m, kJfErrAbort);
+    atomicOr(a.drift + s_seg[tid].m, kDriftUnknown);
   }
   // every warp is past its last access: the TMEM allocation is freed
   if constexpr (kTmem) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -573,9 +581,8 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
     const JfInst* __restrict__ inst, int32_t* __restrict__ counts, int stride, const int32_t* __restrict__ solid,
     const int32_t* __restrict__ rowoff, int32_t* __restrict__ rowcost, int32_t* __restrict__ ovrow,
     int32_t* __restrict__ ovcur, int32_t* __restrict__ cap_out, int fixed_cap, int32_t* __restrict__ band, int CS,
-    unsigned long long* __restrict__ bar, int32_t* __restrict__ drift, int32_t* __restrict__ abort,
-    float4* __restrict__ spill,
-    int64_t nodes, int M) {
+    unsigned long long* __restrict__ bar, int32_t* __restrict__ drift, float4* __restrict__ spill, int64_t nodes,
+    int M) {
   constexpr int kWarps = kScanThreads / 32;
   __shared__ int s_cost[32];
   __shared__ int s_row_cost[kJfMaxBandRows];
@@ -590,7 +597,7 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
   const int segs = (I.nx + 31) >> 5;
   // what a chunk's last substeps may have left in the spill grids
   for (int r = 0; r < 3; ++r)
-    if (drift[m] >> r & 1)
+    if ((drift[m] >> r & 1) || (drift[m] & kDriftUnknown))
       for (int n = tid; n < I.nx * I.ny; n += kScanThreads)
         spill[(int64_t)r * nodes + I.g_off + n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (tid < 32) s_cost[tid] = 0;
@@ -601,7 +608,6 @@ __global__ void __launch_bounds__(kScanThreads) span_scan_kernel(
   __syncthreads();
   if (tid == 0) drift[m] = 0;
   if (tid < 3) bar[tid * M + m] = 0ull;
-  if (tid == 0 && m == 0) *abort = 0;
 
   // lane k sums the cost of candidate k (0 = no cap)
   int cost = 0;
@@ -1014,9 +1020,10 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
     parts.emplace_back((void**)p, bytes);
     bytes += (sizeof(**p) * std::max<size_t>(n, 1) + 255) / 256 * 256;
   };
-  part(&s->d_spill, 3 * (size_t)e->total_nodes);  // the first three are cleared
+  part(&s->d_spill, 3 * (size_t)e->total_nodes);  // the first four are cleared
   part(&s->d_slot, slots);
   part(&s->d_drift, M);
+  part(&s->d_abort, 1);
   const size_t zero_end = bytes;
   part(&s->d_groups, ng);
   part(&s->d_rowoff, M + 1);
@@ -1030,7 +1037,6 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
   part(&s->d_nseg, ng * n_cta);
   part(&s->d_nbar, M);
   part(&s->d_bar, 3 * M);
-  part(&s->d_abort, 1);
   if ((err = cudaMalloc(&s->pool, bytes))) return err;
   for (auto& p : parts) *p.first = (char*)s->pool + p.second;
   const uint32_t first_tag = 1;  // the slots start at 0
@@ -1052,7 +1058,7 @@ cudaError_t jf_span_sort(jf_engine* e) {
   const int stride = e->max_cells + 2;
   span_scan_kernel<<<e->M, kScanThreads, 0, e->stream>>>(
       e->d_inst, e->d_counts, stride, e->d_solid, s->d_rowoff, s->d_rowcost, s->d_ovrow, s->d_ovcur, e->d_cap,
-      e->cell_cap, e->d_band, e->cluster, s->d_bar, s->d_drift, s->d_abort, s->d_spill, e->total_nodes, e->M);
+      e->cell_cap, e->d_band, e->cluster, s->d_bar, s->d_drift, s->d_spill, e->total_nodes, e->M);
   span_cut_kernel<<<(int)s->groups.size(), kScanThreads, 0, e->stream>>>(
       s->d_groups, e->d_inst, s->d_rowoff, s->d_rowcost, s->d_rowpre, s->cap_nodes, s->n_cta, s->threads / 32,
       s->d_fallback, s->d_seg, s->d_nseg, s->d_nbar);
@@ -1089,6 +1095,7 @@ cudaError_t jf_span_launch(jf_engine* e, int K) {
   a.bar = s->d_bar;
   a.drift = s->d_drift;
   a.abort = s->d_abort;
+  a.spin_limit = s->spin_limit;
   a.tag = s->d_tag;
   a.spill = s->d_spill;
   a.slot = s->d_slot;
@@ -1126,3 +1133,11 @@ cudaError_t jf_span_launch(jf_engine* e, int K) {
 // chunk of K substeps adds to it after its last launch.
 uint32_t* jf_span_tag(const jf_engine* e) { return e->span->d_tag; }
 uint32_t jf_span_tag_step(const jf_engine* e, int K) { return (uint32_t)(e->span->groups.size() * K); }
+
+// The poll count after which a wait gives up, 0 for the default.
+void jf_span_set_wait_limit(jf_engine* e, uint32_t polls) { e->span->spin_limit = polls ? polls : kSpinLimit; }
+
+// Lets chunks run again after a wait has given up.
+cudaError_t jf_span_clear_abort(jf_engine* e) {
+  return cudaMemsetAsync(e->span->d_abort, 0, sizeof(int32_t), e->stream);
+}

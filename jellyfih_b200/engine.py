@@ -393,9 +393,18 @@ class Engine:
         return out
 
     def error_flags(self) -> np.ndarray:
+        """Per-instance flags since the last clear, 0 or a sum of JF_ERRFLAG_*: 1 a
+        NaN or Inf in the G2P update, 2 and 4 the same in a differentiable
+        rollout's sums and adjoints, 256 left unfinished because a thread block
+        gave up waiting for another (clear the flags, load it again)."""
         out = np.zeros(self.M, np.int32)
         self._check(self._lib.jf_error_flags(self._h, _ptr(out)))
         return out
 
     def clear_error_flags(self) -> None:
         self._check(self._lib.jf_clear_error_flags(self._h))
+
+    def set_wait_limit(self, polls: int = 0) -> None:
+        """Polls (some 0.7 us each) after which a thread block of the batched path
+        gives up waiting for its neighbours' rows; 0: the default, some 14 s."""
+        self._check(self._lib.jf_set_wait_limit(self._h, int(polls)))
