@@ -208,7 +208,8 @@ template <class R> struct Tile;
 template <> struct Tile<float> {
   int hi[3 * kTileNodes], lo[3 * kTileNodes];
   __device__ __forceinline__ void clear(int e) { hi[e] = lo[e] = 0; }
-  static constexpr float kMax = 1.0f;  // contributions the split holds, |v| below
+  // the split holds contributions up to 1; 1.27 is the largest product of two weights
+  static constexpr float kMax = 0.75f;
   __device__ __forceinline__ void add(int e, float v) {
     constexpr float kMagic = 12582912.0f;  // 1.5 2^23
     const float t = __fadd_rn(__fmul_rn(v, 4194304.0f), kMagic);
@@ -224,7 +225,7 @@ template <> struct Tile<float> {
 template <> struct Tile<double> {
   double acc[3 * kTileNodes];
   __device__ __forceinline__ void clear(int e) { acc[e] = 0.0; }
-  static constexpr double kMax = (double)kFixMax;
+  static constexpr double kMax = 0.75 * (double)kFixMax;  // so that no contribution reaches kFixMax
   __device__ __forceinline__ void add(int e, double v) { atomicAdd(acc + e, v); }
   __device__ __forceinline__ double get(int e) const { return acc[e]; }
 };
@@ -323,11 +324,13 @@ __global__ void __launch_bounds__(kT, sizeof(R) == 4 ? 5 : 1) gf_step(GradArgs<R
   const int entries = 3 * W * H;
   for (int e = threadIdx.x; e < entries; e += blockDim.x) s_acc.clear(e);
   __syncthreads();
-  // a bound on every contribution of the particle: weights are below 1 and node
-  // offsets within 1.5 dx
+  // A bound on every contribution of the particle.  Inside the lower walls (a
+  // stencil coordinate of 0 to 1.5) weights are at most 1.125 an axis and node
+  // offsets within 2 dx; outside them, or with a NaN for a position, it says nothing.
+  const bool inside = valid && st.fx0 >= R(0) && st.fx1 >= R(0);
   const R bound = fabs(sc.mv0) + fabs(sc.mv1) + fabs(sc.mass) +
                   R(2) * I.dx * (fabs(sc.af00) + fabs(sc.af01) + fabs(sc.af10) + fabs(sc.af11));
-  if (valid && bound < Tile<R>::kMax) {
+  if (inside && bound < Tile<R>::kMax) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
 #pragma unroll
