@@ -153,6 +153,13 @@ struct SlotArrays {
   float2* fiber;
 };
 
+// After a synchronised slot-order kernel: whether every slot was in range.
+int check_slots(jf_engine* e) {
+  if (!*e->h_slot_bad) return JF_OK;
+  *e->h_slot_bad = 0;
+  return fail(e, JF_ERR_CUDA, "corrupt slot permutation");
+}
+
 int slot_arrays(jf_engine* e, int m, SlotArrays& a) {
   const size_t n = (size_t)e->inst[m].n_slots;
   if (e->q.xv) {
@@ -394,12 +401,14 @@ int jf_create(const jf_config* cfg, jf_engine** out) {
       (err = alloc(&e->d_grid, g_off)) != cudaSuccess ||
       (err = alloc(&e->d_stats, 6 * (size_t)e->M)) != cudaSuccess ||
       (err = alloc(&e->d_err, e->M)) != cudaSuccess ||
+      (err = cudaHostAlloc((void**)&e->h_slot_bad, sizeof(int32_t), cudaHostAllocMapped)) != cudaSuccess ||
       (err = alloc(&e->d_stage, 8 * (size_t)e->max_slots)) != cudaSuccess ||
       (err = alloc(&e->d_stage_i, 2 * (size_t)e->max_slots)) != cudaSuccess ||
       (err = alloc(&e->d_fit, 6 * (size_t)e->M)) != cudaSuccess ||
       (err = alloc(&e->d_fit_f, e->M)) != cudaSuccess ||
       (err = alloc(&e->d_fit_i, e->M)) != cudaSuccess)
     return bail(JF_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(err));
+  *e->h_slot_bad = 0;
   if (e->path == JF_PATH_BATCHED) {
     if ((err = alloc_particles(e->q, p_off)) != cudaSuccess ||
         (err = alloc(&e->d_keys, p_off)) != cudaSuccess ||
@@ -465,6 +474,7 @@ int jf_destroy(jf_engine* e) {
   cudaFree(e->d_rank); cudaFree(e->d_ovlist); cudaFree(e->d_ovband); cudaFree(e->d_ovcur);
   cudaFree(e->d_band); cudaFree(e->d_cap); cudaFree(e->d_order); cudaFree(e->d_brow); cudaFree(e->d_solid); cudaFree(e->d_ep); cudaFree(e->d_ep_mat);
   cudaFree(e->d_ep_stats); cudaFree(e->d_grid); cudaFree(e->d_stats); cudaFree(e->d_err);
+  cudaFreeHost(e->h_slot_bad);
   cudaFree(e->d_stage); cudaFree(e->d_stage_i); cudaFree(e->d_path);
   cudaFree(e->d_fit); cudaFree(e->d_fit_f); cudaFree(e->d_fit_i); cudaFree(e->d_time);
   cudaFree(e->d_frame); cudaFree(e->d_vort); cudaFree(e->d_hue); cudaFree(e->d_slot_stage); cudaFree(e->d_tank_stage);
@@ -961,7 +971,7 @@ int jf_grad_positions(jf_engine* e, int32_t m, float* dx0) {
   JF_CK(jf_grad_x0_launch(e, m, a.x), "position adjoint");
   JF_CK(cudaMemcpyAsync(dx0, a.x, sizeof(float2) * n, cudaMemcpyDeviceToHost, e->stream), "read position adjoint");
   JF_CK(cudaStreamSynchronize(e->stream), "position adjoint sync");
-  return JF_OK;
+  return check_slots(e);
 }
 
 int jf_read_particles(jf_engine* e, int32_t m, float* x, float* v, float* C, float* F, int32_t* material,
@@ -981,7 +991,7 @@ int jf_read_particles(jf_engine* e, int32_t m, float* x, float* v, float* C, flo
   for (const auto& p : parts)
     if (p.to) JF_CK(cudaMemcpyAsync(p.to, p.from, p.bytes, cudaMemcpyDeviceToHost, e->stream), "read particles");
   JF_CK(cudaStreamSynchronize(e->stream), "read particles sync");
-  return JF_OK;
+  return check_slots(e);
 }
 
 int jf_write_particles(jf_engine* e, int32_t m, const float* x, const float* v, const float* C, const float* F,
@@ -1002,6 +1012,7 @@ int jf_write_particles(jf_engine* e, int32_t m, const float* x, const float* v, 
                              Jp ? a.Jp : nullptr, glow ? a.glow : nullptr),
           "engine order");
     JF_CK(cudaStreamSynchronize(e->stream), "write particles sync");
+    if ((rc = check_slots(e))) return rc;
   }
   if (x) e->sorted = false;
   return JF_OK;

@@ -1495,18 +1495,24 @@ cudaError_t step_impl(jf_engine* e, int64_t steps, int32_t K, const int32_t* bod
 // Position adjoint of instance I in slot order, rounded to FP32.
 template <class R>
 __global__ void x0_kernel(JfInst I, const V4<R>* __restrict__ lxv, const int32_t* __restrict__ slot,
-                          float2* __restrict__ out) {
+                          float2* __restrict__ out, int32_t* bad) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= I.n_slots) return;
   const int64_t g = I.p_off + k;
+  const int s = slot[g];
+  if ((unsigned)s >= (unsigned)I.n_slots) {
+    *bad = 1;
+    return;
+  }
   const V4<R> a = lxv[g];
-  out[slot[g]] = make_float2((float)a.x, (float)a.y);
+  out[s] = make_float2((float)a.x, (float)a.y);
 }
 
 template <class R>
 cudaError_t x0_launch(jf_engine* e, int m, float2* d_out) {
   const JfInst& I = e->inst[m];
-  x0_kernel<R><<<(I.n_slots + kT - 1) / kT, kT, 0, e->stream>>>(I, bufs<R>(e).lxv, e->p.slot, d_out);
+  x0_kernel<R><<<(I.n_slots + kT - 1) / kT, kT, 0, e->stream>>>(I, bufs<R>(e).lxv, e->p.slot, d_out,
+                                                                e->h_slot_bad);
   e->launches += 1;
   return cudaGetLastError();
 }

@@ -217,13 +217,18 @@ __global__ void glow_to_slot_kernel(JfInst I, const float* __restrict__ glow,
 // Engine order -> slot order: engine position k holds slot slot[k], so that a
 // read gathers on the device and every field leaves in one copy to the
 // caller's array (a host-side permutation of 64 B per slot took 2-3 ms of an
-// 80K-slot read).  Reads are coalesced; the scattered writes stay in L2.
+// 80K-slot read).  Reads are coalesced; the scattered writes stay in L2.  A slot
+// outside the instance is left out and reported in *bad (host memory).
 __global__ void slots_out_kernel(JfInst I, JfParticles p, float2* x, float2* v, float4* C, float4* F, int32_t* mat,
-                                 float* Jp, float* glow, float2* fiber) {
+                                 float* Jp, float* glow, float2* fiber, int32_t* bad) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= I.n_slots) return;
   const int64_t g = I.p_off + k;
   const int s = p.slot[g];
+  if ((unsigned)s >= (unsigned)I.n_slots) {
+    *bad = 1;
+    return;
+  }
   const float4 a = p.xv[g];
   x[s] = make_float2(a.x, a.y);
   v[s] = make_float2(a.z, a.w);
@@ -237,11 +242,15 @@ __global__ void slots_out_kernel(JfInst I, JfParticles p, float2* x, float2* v, 
 
 // Slot order -> engine order, the fields that are given.
 __global__ void slots_in_kernel(JfInst I, JfParticles p, const float2* x, const float2* v, const float4* C,
-                                const float4* F, const float* Jp, const float* glow) {
+                                const float4* F, const float* Jp, const float* glow, int32_t* bad) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= I.n_slots) return;
   const int64_t g = I.p_off + k;
   const int s = p.slot[g];
+  if ((unsigned)s >= (unsigned)I.n_slots) {
+    *bad = 1;
+    return;
+  }
   if (x || v) {
     float4 a = p.xv[g];
     if (x) {
@@ -396,7 +405,8 @@ cudaError_t jf_rows_launch(jf_engine* e, const double* d_before, const double* d
 cudaError_t jf_slots_out_launch(jf_engine* e, int m, float2* x, float2* v, float4* C, float4* F, int32_t* mat,
                                 float* Jp, float* glow, float2* fiber) {
   const JfInst& I = e->inst[m];
-  slots_out_kernel<<<blocks_for(I.n_slots), kThreads, 0, e->stream>>>(I, e->p, x, v, C, F, mat, Jp, glow, fiber);
+  slots_out_kernel<<<blocks_for(I.n_slots), kThreads, 0, e->stream>>>(I, e->p, x, v, C, F, mat, Jp, glow, fiber,
+                                                                     e->h_slot_bad);
   e->launches += 1;
   return cudaGetLastError();
 }
@@ -404,7 +414,7 @@ cudaError_t jf_slots_out_launch(jf_engine* e, int m, float2* x, float2* v, float
 cudaError_t jf_slots_in_launch(jf_engine* e, int m, const float2* x, const float2* v, const float4* C,
                                const float4* F, const float* Jp, const float* glow) {
   const JfInst& I = e->inst[m];
-  slots_in_kernel<<<blocks_for(I.n_slots), kThreads, 0, e->stream>>>(I, e->p, x, v, C, F, Jp, glow);
+  slots_in_kernel<<<blocks_for(I.n_slots), kThreads, 0, e->stream>>>(I, e->p, x, v, C, F, Jp, glow, e->h_slot_bad);
   e->launches += 1;
   return cudaGetLastError();
 }
