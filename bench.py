@@ -645,6 +645,7 @@ def run_ours(args):
                     block_threads=args.block)
     stream = torch.cuda.Stream()
     engine.set_stream(stream)
+    spans, layout = engine.spans(), engine.layout()
     load_all(engine, inputs)
     engine.time = 0.0
 
@@ -686,7 +687,7 @@ def run_ours(args):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": (tpps * live * chunk_substeps) if tpps else None,
-                "kernel": "span_kernel", "algorithmic_bytes_per_launch": bytes_per_launch,
+                "kernel": "span_kernel" if spans else "chunk_kernel", "algorithmic_bytes_per_launch": bytes_per_launch,
                 "mean_launch_ms": mean_launch_s * 1e3, "launches": kt["step_launches"],
                 "step_kernel_share": kt["step_ms"] / ms if ms > 0 else None,
                 "scatter_paths": paths,
@@ -778,7 +779,9 @@ def run_ours(args):
                                        f"FP32, {S} substeps per step",
                            "instances_per_gpu": M, "slots": args.slots, "live_particles": int(live_total),
                            "substeps_per_step": S, "resort_interval": args.resort,
-                           "layout": "spans of grid rows, one CTA per SM", "block_threads": args.block or 512,
+                           "layout": f"{spans['ctas']} spans of grid rows, {spans['launches']} launch(es) per chunk"
+                           if spans else f"clusters of {layout['cluster_size']}",
+                           "block_threads": (spans or layout)["block_threads"],
                            "l2": "inputs larger than L2: particle state plus sort buffers ~260 MB per GPU",
                            "path": "batched"},
                 "roofline": roofline, "clocks": clocks.summary(), "gpu_launches": gpu_launches,

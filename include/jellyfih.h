@@ -322,6 +322,15 @@ int jf_path_counts(jf_engine* e, int64_t* out, int32_t reset);
  * layout is Taichi's). */
 int jf_get_layout(const jf_engine* e, int32_t* cluster_size, int32_t* block_threads);
 
+/* How the batch runs as spans.  info[4]: launches per chunk of substeps, CTAs
+ * of the largest of them, threads per CTA, nodes that a CTA's shared-memory
+ * windows hold; all zero for an engine that runs as clusters or on the plain
+ * path.  The bands of grid rows as the latest re-sort cut them go to
+ * bands[capacity][5]: launch, CTA, instance, first row, end row; *n_bands is how
+ * many there are (0 before the first re-sort), also where the capacity is less.
+ * bands may be NULL with a capacity of 0.  No counterpart in the reference. */
+int jf_get_spans(jf_engine* e, int32_t* info, int32_t* bands, int32_t capacity, int32_t* n_bands);
+
 /* Largest grid, in nodes (n_grid * n_grid_y), jf_substep_noalloc accepts. */
 #define JF_NOALLOC_MAX_NODES 32768
 

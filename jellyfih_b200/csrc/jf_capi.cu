@@ -1095,6 +1095,21 @@ int jf_get_layout(const jf_engine* e, int32_t* cluster_size, int32_t* block_thre
   return JF_OK;
 }
 
+int jf_get_spans(jf_engine* e, int32_t* info, int32_t* bands, int32_t capacity, int32_t* n_bands) {
+  if (check_engine(e) || need_args(e, info && n_bands && (bands || capacity <= 0), "jf_get_spans: info, n_bands, bands"))
+    return JF_ERR_INVALID;
+  int rc = set_device(e);
+  if (rc) return rc;
+  std::fill(info, info + 4, 0);
+  *n_bands = 0;
+  if (!e->span) return JF_OK;
+  std::vector<int32_t> b;
+  JF_CK(jf_span_info(e, info, b), "read spans");
+  *n_bands = (int32_t)(b.size() / 5);
+  std::copy_n(b.begin(), 5 * (size_t)std::max(0, std::min(capacity, *n_bands)), bands);
+  return JF_OK;
+}
+
 int jf_set_kernel_timing(jf_engine* e, int32_t enable) {
   if (check_engine(e)) return JF_ERR_INVALID;
   int rc = set_device(e);

@@ -153,6 +153,8 @@ cudaError_t jf_span_setup(jf_engine* e, int threads);
 cudaError_t jf_span_sort(jf_engine* e);
 cudaError_t jf_span_launch(jf_engine* e, int K);
 void jf_span_free(jf_engine* e);
+// info[4] and bands (5 values each) of jf_get_spans.
+cudaError_t jf_span_info(jf_engine* e, int32_t* info, std::vector<int32_t>& bands);
 void jf_span_set_wait_limit(jf_engine* e, uint32_t polls);
 cudaError_t jf_span_clear_abort(jf_engine* e);
 uint32_t* jf_span_tag(const jf_engine* e);

@@ -1020,10 +1020,11 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
     parts.emplace_back((void**)p, bytes);
     bytes += (sizeof(**p) * std::max<size_t>(n, 1) + 255) / 256 * 256;
   };
-  part(&s->d_spill, 3 * (size_t)e->total_nodes);  // the first four are cleared
+  part(&s->d_spill, 3 * (size_t)e->total_nodes);  // the first five are cleared
   part(&s->d_slot, slots);
   part(&s->d_drift, M);
   part(&s->d_abort, 1);
+  part(&s->d_nseg, ng * n_cta);
   const size_t zero_end = bytes;
   part(&s->d_groups, ng);
   part(&s->d_rowoff, M + 1);
@@ -1034,7 +1035,6 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
   part(&s->d_ovrow, rows + M);
   part(&s->d_ovcur, rows);
   part(&s->d_seg, ng * n_cta * kMaxSeg);
-  part(&s->d_nseg, ng * n_cta);
   part(&s->d_nbar, M);
   part(&s->d_bar, 3 * M);
   if ((err = cudaMalloc(&s->pool, bytes))) return err;
@@ -1140,4 +1140,27 @@ void jf_span_set_wait_limit(jf_engine* e, uint32_t polls) { e->span->spin_limit 
 // Lets chunks run again after a wait has given up.
 cudaError_t jf_span_clear_abort(jf_engine* e) {
   return cudaMemsetAsync(e->span->d_abort, 0, sizeof(int32_t), e->stream);
+}
+
+// The layout: launches, CTAs, threads and window nodes, and the bands of the latest re-sort.
+cudaError_t jf_span_info(jf_engine* e, int32_t* info, std::vector<int32_t>& bands) {
+  const JfSpan* s = e->span;
+  info[0] = (int32_t)s->groups.size();
+  info[1] = s->n_cta;
+  info[2] = s->threads;
+  info[3] = s->cap_nodes;
+  const size_t n = s->groups.size() * s->n_cta;
+  std::vector<int32_t> nseg(n);
+  std::vector<int4> seg(n * kMaxSeg);
+  cudaError_t err;
+  if ((err = cudaMemcpyAsync(nseg.data(), s->d_nseg, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, e->stream)) ||
+      (err = cudaMemcpyAsync(seg.data(), s->d_seg, sizeof(int4) * n * kMaxSeg, cudaMemcpyDeviceToHost, e->stream)) ||
+      (err = cudaStreamSynchronize(e->stream)))
+    return err;
+  for (size_t c = 0; c < n; ++c)
+    for (int k = 0; k < nseg[c]; ++k) {
+      const int4 q = seg[c * kMaxSeg + k];
+      bands.insert(bands.end(), {(int32_t)(c / s->n_cta), (int32_t)(c % s->n_cta), q.x, q.y, q.z});
+    }
+  return cudaSuccess;
 }

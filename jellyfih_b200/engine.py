@@ -152,6 +152,20 @@ class Engine:
         self._check(self._lib.jf_get_layout(self._h, _ptr(cs), _ptr(bt)))
         return {"cluster_size": int(cs[0]), "block_threads": int(bt[0])}
 
+    def spans(self) -> dict | None:
+        """How the batch runs as spans: launches per chunk, CTAs of the largest,
+        threads per CTA, nodes of a CTA's windows, and the bands (launch, CTA,
+        instance, first row, end row) of the latest re-sort.  None where it runs
+        as clusters or on the plain path."""
+        info, n = np.zeros(4, np.int32), np.zeros(1, np.int32)
+        self._check(self._lib.jf_get_spans(self._h, _ptr(info), None, 0, _ptr(n)))
+        if not info[0]:
+            return None
+        bands = np.zeros((int(n[0]), 5), np.int32)
+        self._check(self._lib.jf_get_spans(self._h, _ptr(info), _ptr(bands), len(bands), _ptr(n)))
+        return {"launches": int(info[0]), "ctas": int(info[1]), "block_threads": int(info[2]),
+                "window_nodes": int(info[3]), "bands": bands}
+
     def set_stream(self, stream) -> None:
         """Queue work on ``stream`` (a cudaStream_t as int, or a torch.cuda.Stream)."""
         handle = getattr(stream, "cuda_stream", stream)
