@@ -97,7 +97,8 @@ const char* jf_last_error(const jf_engine* e);
 const char* jf_version(void);
 
 /* Stream the engine queues work on (a cudaStream_t); NULL restores the
- * engine's own stream. */
+ * engine's own stream.  A stream of a green context, which has some of the
+ * device's SMs, gets a batched layout of its own for them. */
 int jf_set_stream(jf_engine* e, void* stream);
 
 /* Reset instance `m` from host arrays of n <= n_slots particles

@@ -439,7 +439,8 @@ int jf_create(const jf_config* cfg, jf_engine** out) {
     if (active == 0)
       return bail(JF_ERR_UNSUPPORTED, "clusters of " + std::to_string(e->cluster) + " CTAs cannot be scheduled");
     // without a cluster size asked for, the batch runs as one span of rows per SM where it can
-    if (cfg->cluster_size == 0 && (err = jf_span_setup(e, cfg->block_threads)) != cudaSuccess)
+    e->auto_layout = cfg->cluster_size == 0;
+    if (e->auto_layout && (err = jf_span_setup(e, cfg->block_threads)) != cudaSuccess)
       return bail(JF_ERR_CUDA, std::string("span set-up: ") + cudaGetErrorString(err));
   }
   if (cudaMemcpy(e->d_inst, e->inst.data(), sizeof(JfInst) * e->M, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -500,6 +501,7 @@ int jf_set_stream(jf_engine* e, void* stream) {
     JF_CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     e->own_stream = true;
   }
+  if (e->auto_layout) JF_CK(jf_span_follow_stream(e), "span set-up");
   return JF_OK;
 }
 

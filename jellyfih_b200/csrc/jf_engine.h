@@ -105,6 +105,9 @@ struct jf_engine {
   std::string err;
 
   JfSpan* span = nullptr;          // batched path: spans over all SMs (jf_span.cu); null: one cluster per instance
+  bool auto_layout = false;        // no cluster size was asked for: spans where the batch suits them
+  int32_t span_threads = 0;        // CTA size asked for, 0 = automatic
+  int32_t span_sms = 0;            // SMs that the layout is made for
   JfGrad* grad = nullptr;          // differentiable rollout buffers (jf_grad.cu)
   // headless renderer (jf_render.cu)
   float4* d_frame = nullptr;       // frame_res^2 pixels (r, g, b, unused), row py = frame row
@@ -150,6 +153,8 @@ size_t jf_batched_smem_bytes(const jf_engine* e);
 // cluster size.
 // threads: CTA size asked for, 0 = automatic.
 cudaError_t jf_span_setup(jf_engine* e, int threads);
+// After a change of e->stream: the layout for the SMs that the new one may use.
+cudaError_t jf_span_follow_stream(jf_engine* e);
 cudaError_t jf_span_sort(jf_engine* e);
 cudaError_t jf_span_launch(jf_engine* e, int K);
 void jf_span_free(jf_engine* e);

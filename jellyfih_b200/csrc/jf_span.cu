@@ -36,6 +36,8 @@
 // flag stays up until jf_clear_error_flags: what is queued behind the chunk
 // returns at once, so that the time of a run whose waits run out is bounded by
 // one of them, and sets the same error flag on the instances it leaves alone.
+#include <cuda.h>
+
 #include <algorithm>
 #include <utility>
 #include <vector>
@@ -892,6 +894,29 @@ SpanKernel span_kernel_for(const jf_engine* e, int threads) {
                 : (glow ? span_kernel<false, false, true> : span_kernel<false, false, false>);
 }
 
+// SMs that kernels on the engine's stream may use: fewer than the device's
+// where the stream belongs to a green context.
+int sms_of_stream(const jf_engine* e) {
+  int n_sm = 0;
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, e->device);
+  CUresult (*of_stream)(CUstream, CUgreenCtx*) = nullptr;
+  CUresult (*resource)(CUgreenCtx, CUdevResource*, CUdevResourceType) = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  if (cudaGetDriverEntryPointByVersion("cuStreamGetGreenCtx", (void**)&of_stream, 12040, cudaEnableDefault, &found) !=
+          cudaSuccess || !of_stream ||
+      cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", (void**)&resource, 12040, cudaEnableDefault,
+                                       &found) != cudaSuccess || !resource) {
+    cudaGetLastError();  // a driver older than green contexts
+    return n_sm;
+  }
+  CUgreenCtx green = nullptr;
+  CUdevResource r;
+  if (of_stream((CUstream)e->stream, &green) != CUDA_SUCCESS || !green ||
+      resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+    return n_sm;
+  return std::min(n_sm, (int)r.sm.smCount);
+}
+
 // Spans of the group by window size alone; false when n_cta spans do not do.
 bool fill_cuts(const jf_engine* e, const SpanGroup& g, const std::vector<int32_t>& rowoff, int cap_nodes,
                std::vector<int32_t>& cuts) {
@@ -935,9 +960,10 @@ void jf_span_free(jf_engine* e) {
 // (the kernel's constants are launch parameters), rows too wide for a band of
 // 4 rows and its halo, or a device without cooperative launches.
 cudaError_t jf_span_setup(jf_engine* e, int threads) {
+  int n_sm = sms_of_stream(e), coop = 0;
+  e->span_threads = threads;
+  e->span_sms = n_sm;
   if (threads == 0) threads = kSpanThreads;
-  int n_sm = 0, coop = 0;
-  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, e->device);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->device);
   if (!coop || n_sm < 1) return cudaSuccess;
   n_sm = std::min(n_sm, kScanThreads);
@@ -1049,6 +1075,26 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
       (err = cudaMemcpyAsync(s->d_tag, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice, e->stream)))
     return err;
   return cudaStreamSynchronize(e->stream);
+}
+
+// One CTA per SM is what the waits between CTAs stand on, so that a stream with
+// other SMs takes spans of its own (or clusters, where these do not fit it).
+cudaError_t jf_span_follow_stream(jf_engine* e) {
+  if (sms_of_stream(e) == e->span_sms) return cudaSuccess;
+  uint32_t limit = kSpinLimit;
+  int32_t abort = 0;
+  cudaError_t err = cudaSuccess;
+  if (e->span) {
+    limit = e->span->spin_limit;
+    if ((err = cudaMemcpy(&abort, e->span->d_abort, sizeof(abort), cudaMemcpyDeviceToHost))) return err;
+  }
+  if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);  // its launches are those of the old layout
+  e->graph_exec = nullptr;
+  jf_span_free(e);
+  e->sorted = false;
+  if ((err = jf_span_setup(e, e->span_threads)) || !e->span) return err;
+  e->span->spin_limit = limit;
+  return abort ? cudaMemcpy(e->span->d_abort, &abort, sizeof(abort), cudaMemcpyHostToDevice) : cudaSuccess;
 }
 
 // The part of a re-sort after the cell keys: bins, spans, and the particles
