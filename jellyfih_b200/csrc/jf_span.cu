@@ -1,16 +1,16 @@
 // Batched path, spans: the grid rows of all instances, one instance after the
-// other, are cut into one contiguous span of about equal cost per SM at every
-// re-sort, and one cooperative launch per chunk of substeps advances them all,
-// one CTA per span.  A CTA owns the bands of rows (one per instance that its
-// span touches) and keeps them, plus a halo, in shared memory for the whole
-// chunk.
+// other, are cut into contiguous spans of about equal cost at every re-sort, one
+// per SM where there are four rows for each, and one cooperative launch per
+// chunk of substeps advances them all, one CTA per span.  A CTA owns the bands
+// of rows (one per instance that its span touches) and keeps them, plus a halo,
+// in shared memory for the whole chunk.
 //
 // Why spans and not one thread-block cluster per instance: clusters are placed
 // per GPC, so that at one CTA per SM only 33 clusters of 4, 15 of 8 or 7 of 16
 // fit a B200 (cudaOccupancyMaxActiveClusters): 32 instances use 128 of the 148
 // SMs, and 16 instances on clusters of 8 or 8 on clusters of 16 take two
-// waves.  Spans use every SM at every batch size, and an instance may share an
-// SM with the next one.
+// waves.  Spans use every SM from 592 rows on (five tanks of 128; one tank
+// takes 32), and an instance may share an SM with the next one.
 //
 // One pass over a CTA's particles fuses G2P of substep s-1 with P2G of substep
 // s (mpm_sim.py:312-333 then :168-271).  Neighbouring bands of an instance
@@ -76,8 +76,10 @@ constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 3072;  // static shared variables of the kernel, rounded up
 // Shared memory and L1 share an SM's 256 KB: larger windows slow the particle
 // loads, so that larger batches run as several groups of instances, one launch
-// after the other, whose equal shares of the rows stay within this size.  The
-// windows may take up to 8/5 of it where bands of equal cost differ in rows.
+// after the other, whose equal shares of the rows stay within this size.  A
+// window may take 8/5 of the largest share, as bands of equal cost differ in
+// rows; up to all of shared memory where one instance's share is already over
+// the size, or where the rows do not fit their CTAs otherwise.
 // Measured on 48 instances of 40K to 120K particles on 128^2 beside 16 of 128K
 // on 128x256 (us per substep; shares of 200, 109, 80 and 65 KB): 1 group 325,
 // 2: 293, 3: 273, 4: 287; at 5/4 of the share 302 and 282 for 2 and 3 (some
