@@ -189,7 +189,7 @@ def traffic_per_particle_step():
             h.update(f.read())
     if h.hexdigest()[:16] != d.get("kernel_sources_sha256_16"):
         return None, d
-    return d.get("chunk_kernel_dram_bytes_per_live_particle_substep"), d
+    return d.get("dram_bytes_per_live_particle_substep"), d
 
 
 def cpu_baseline(inputs, target_s=12.0):
@@ -696,7 +696,7 @@ def run_ours(args):
         # the kernel changed since the ncu measurement: no traffic figure for this
         # source, but the last measured one, scaled to this launch, and the sources
         # it belongs to
-        last = trec.get("chunk_kernel_dram_bytes_per_live_particle_substep")
+        last = trec.get("dram_bytes_per_live_particle_substep")
         roofline["traffic_last_measured"] = {
             "bytes_per_launch": last * live * chunk_substeps if last else None,
             "kernel_sources_sha256_16": trec.get("kernel_sources_sha256_16"),
