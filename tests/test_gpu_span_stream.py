@@ -47,3 +47,36 @@ def test_spans_follow_a_stream_with_fewer_sms(count, sms):
     driver.cuGreenCtxDestroy(green)
     # the bound that a chunk has against the clusters in test_gpu_span.py
     assert np.abs(few - want).max() <= 1e-6 and np.abs(again - want).max() <= 1e-6
+
+
+def test_engines_side_by_side_on_threads_and_streams():
+    """Three engines, whose launches each take every SM, from three threads at
+    once: a cooperative launch is placed whole, so that no wait runs out, and the
+    rows are those of a run alone (the bound of a chunk, as above)."""
+    import threading
+
+    from jellyfih_b200 import Engine, InstanceSpec, tank
+    tanks = [tank.fill_tank(g, 80000)[:3] for g in tank.gaussian_genomes(8, 5)]
+    engines = [Engine([InstanceSpec(80000)] * 8) for _ in range(3)]
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1, 0)]
+    got = [[] for _ in engines]
+
+    def run(k, times):
+        for _ in range(times):
+            for m, t in enumerate(tanks):
+                engines[k].load(m, *t)
+            got[k].append(engines[k].run_headless(192))
+    for e, s in zip(engines, streams):
+        e.set_stream(s)
+        e.set_wait_limit(3000000)  # some two seconds
+    run(0, 1)
+    want = got[0].pop()
+    threads = [threading.Thread(target=run, args=(k, 6)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for e, rows in zip(engines, got):
+        assert len(rows) == 6 and not e.error_flags().any()
+        assert max(np.abs(r - want).max() for r in rows) <= 1e-6
+        e.close()
