@@ -76,7 +76,7 @@ typedef struct {
                                            (ceil(n_grid_y / cluster size)), else 512 */
   int32_t cluster_size;                 /* batched: one cluster of this many CTAs (1..16) per
                                            instance.  0 = automatic: the grid rows of the whole
-                                           batch cut into one span of equal cost per SM, or
+                                           batch cut into spans of equal cost, up to one per SM, or
                                            clusters where the batch does not suit that (instances
                                            of different n_grid, n_grid_y > 1024) */
   int32_t cell_cap;                     /* batched: particles a cell lane accumulates per substep;

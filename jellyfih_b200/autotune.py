@@ -5,7 +5,7 @@ own batch.
 Candidates are the kernel layouts (threads per CTA: fewer warps per SM leave
 more registers and L1 per warp but hide less latency; the cell cap chosen by
 the sort's cost model at every re-sort, or fixed), the batch's layout (cluster
-size 0: one span of grid rows per SM; else the cluster sizes whose
+size 0: spans of grid rows, up to one per SM; else the cluster sizes whose
 shared-memory window fits: more CTAs per instance give it more SMs but more
 halo rows) and the re-sort intervals (longer intervals
 amortise the counting sort; particles that drift out of their cell's register

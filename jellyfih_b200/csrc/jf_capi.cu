@@ -438,7 +438,7 @@ int jf_create(const jf_config* cfg, jf_engine** out) {
     jf_batched_max_active_clusters(e, e->cluster, &active);
     if (active == 0)
       return bail(JF_ERR_UNSUPPORTED, "clusters of " + std::to_string(e->cluster) + " CTAs cannot be scheduled");
-    // without a cluster size asked for, the batch runs as one span of rows per SM where it can
+    // without a cluster size asked for, the batch runs as spans of rows, up to one per SM, where it can
     e->auto_layout = cfg->cluster_size == 0;
     if (e->auto_layout && (err = jf_span_setup(e, cfg->block_threads)) != cudaSuccess)
       return bail(JF_ERR_CUDA, std::string("span set-up: ") + cudaGetErrorString(err));

@@ -1065,7 +1065,10 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
   part(&s->d_seg, ng * n_cta * kMaxSeg);
   part(&s->d_nbar, M);
   part(&s->d_bar, 3 * M);
-  if ((err = cudaMalloc(&s->pool, bytes))) return err;
+  if ((err = cudaMalloc(&s->pool, bytes))) {
+    jf_span_free(e);
+    return err;
+  }
   for (auto& p : parts) *p.first = (char*)s->pool + p.second;
   const uint32_t first_tag = 1;  // the slots start at 0
   if ((err = cudaMemsetAsync(s->pool, 0, zero_end, e->stream)) ||
@@ -1074,9 +1077,10 @@ cudaError_t jf_span_setup(jf_engine* e, int threads) {
                              e->stream)) ||
       (err = cudaMemcpyAsync(s->d_fallback, table.data(), sizeof(int32_t) * table.size(), cudaMemcpyHostToDevice,
                              e->stream)) ||
-      (err = cudaMemcpyAsync(s->d_tag, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice, e->stream)))
-    return err;
-  return cudaStreamSynchronize(e->stream);
+      (err = cudaMemcpyAsync(s->d_tag, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice, e->stream)) ||
+      (err = cudaStreamSynchronize(e->stream)))
+    jf_span_free(e);  // no half-made layout is left to a later launch
+  return err;
 }
 
 // One CTA per SM is what the waits between CTAs stand on, so that a stream with

@@ -52,7 +52,7 @@ class Engine:
     """A batch of independent MLS-MPM instances on one GPU.
 
     ``path='batched'`` advances every instance in one persistent launch per
-    chunk (the batch's grid rows cut into one span per SM, or, with a
+    chunk (the batch's grid rows cut into spans, up to one per SM, or, with a
     ``cluster_size``, one thread-block cluster per instance); ``path='plain'`` launches clear / P2G / grid update / G2P per
     instance and substep, as the reference's substep() offloads do.
     ``axisym=True`` runs the axisymmetric (r, z) substep of JELLY_AXISYM=1
