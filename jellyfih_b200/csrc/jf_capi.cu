@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <utility>
@@ -152,6 +153,39 @@ struct SlotArrays {
   float *Jp, *glow;
   float2* fiber;
 };
+
+// A word per engine in one page of the library that the GPU may write, so that a
+// kernel's complaint is there after the synchronisation that the call makes
+// anyway: a 4-byte copy beside it is 12 us of a 50 us write.  The page is
+// registered once (1 to 5 ms, ten times a small engine's creation), and again
+// after a device reset.  Engines beyond the page share its last word.
+alignas(4096) int32_t g_words[1024];
+bool g_taken[1024];
+std::mutex g_words_mutex;
+
+cudaError_t take_word(jf_engine* e) {
+  std::lock_guard<std::mutex> lock(g_words_mutex);
+  void* d = nullptr;
+  if (cudaHostGetDevicePointer(&d, g_words, 0) != cudaSuccess) {
+    cudaGetLastError();  // not registered
+    cudaError_t err = cudaHostRegister(g_words, sizeof(g_words), cudaHostRegisterPortable | cudaHostRegisterMapped);
+    if (err == cudaSuccess) err = cudaHostGetDevicePointer(&d, g_words, 0);
+    if (err != cudaSuccess) return err;
+  }
+  int k = 0;
+  while (k < 1023 && g_taken[k]) ++k;
+  g_taken[k] = true;
+  g_words[k] = 0;
+  e->h_slot_bad = g_words + k;
+  e->d_slot_bad = (int32_t*)d + k;
+  return cudaSuccess;
+}
+
+void give_word(jf_engine* e) {
+  if (!e->h_slot_bad) return;
+  std::lock_guard<std::mutex> lock(g_words_mutex);
+  g_taken[e->h_slot_bad - g_words] = false;
+}
 
 // After a synchronised slot-order kernel: whether every slot was in range.
 int check_slots(jf_engine* e) {
@@ -401,14 +435,13 @@ int jf_create(const jf_config* cfg, jf_engine** out) {
       (err = alloc(&e->d_grid, g_off)) != cudaSuccess ||
       (err = alloc(&e->d_stats, 6 * (size_t)e->M)) != cudaSuccess ||
       (err = alloc(&e->d_err, e->M)) != cudaSuccess ||
-      (err = cudaHostAlloc((void**)&e->h_slot_bad, sizeof(int32_t), cudaHostAllocMapped)) != cudaSuccess ||
+      (err = take_word(e)) != cudaSuccess ||
       (err = alloc(&e->d_stage, 8 * (size_t)e->max_slots)) != cudaSuccess ||
       (err = alloc(&e->d_stage_i, 2 * (size_t)e->max_slots)) != cudaSuccess ||
       (err = alloc(&e->d_fit, 6 * (size_t)e->M)) != cudaSuccess ||
       (err = alloc(&e->d_fit_f, e->M)) != cudaSuccess ||
       (err = alloc(&e->d_fit_i, e->M)) != cudaSuccess)
     return bail(JF_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(err));
-  *e->h_slot_bad = 0;
   if (e->path == JF_PATH_BATCHED) {
     if ((err = alloc_particles(e->q, p_off)) != cudaSuccess ||
         (err = alloc(&e->d_keys, p_off)) != cudaSuccess ||
@@ -475,7 +508,7 @@ int jf_destroy(jf_engine* e) {
   cudaFree(e->d_rank); cudaFree(e->d_ovlist); cudaFree(e->d_ovband); cudaFree(e->d_ovcur);
   cudaFree(e->d_band); cudaFree(e->d_cap); cudaFree(e->d_order); cudaFree(e->d_brow); cudaFree(e->d_solid); cudaFree(e->d_ep); cudaFree(e->d_ep_mat);
   cudaFree(e->d_ep_stats); cudaFree(e->d_grid); cudaFree(e->d_stats); cudaFree(e->d_err);
-  cudaFreeHost(e->h_slot_bad);
+  give_word(e);
   cudaFree(e->d_stage); cudaFree(e->d_stage_i); cudaFree(e->d_path);
   cudaFree(e->d_fit); cudaFree(e->d_fit_f); cudaFree(e->d_fit_i); cudaFree(e->d_time);
   cudaFree(e->d_frame); cudaFree(e->d_vort); cudaFree(e->d_hue); cudaFree(e->d_slot_stage); cudaFree(e->d_tank_stage);

@@ -84,7 +84,8 @@ struct jf_engine {
   int32_t* d_stage_i = nullptr;    // staging for ints (max_slots * 2)
   float* d_slot_stage = nullptr;   // packed frames; plain path: slot-order reads and writes
   size_t slot_stage_floats = 0;
-  int32_t* h_slot_bad = nullptr;   // mapped host memory: a slot-order kernel met a slot out of range
+  volatile int32_t* h_slot_bad = nullptr;  // a slot-order kernel met a slot out of range: a word of host memory
+  int32_t* d_slot_bad = nullptr;           // and its device address
   double* d_tank_stage = nullptr;  // tank fill: robot positions, lattice flags and counts
   size_t tank_stage_bytes = 0;
   unsigned long long* d_path = nullptr;  // batched path counters (see jf_path_counts)

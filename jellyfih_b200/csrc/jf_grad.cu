@@ -1512,7 +1512,7 @@ template <class R>
 cudaError_t x0_launch(jf_engine* e, int m, float2* d_out) {
   const JfInst& I = e->inst[m];
   x0_kernel<R><<<(I.n_slots + kT - 1) / kT, kT, 0, e->stream>>>(I, bufs<R>(e).lxv, e->p.slot, d_out,
-                                                                e->h_slot_bad);
+                                                                e->d_slot_bad);
   e->launches += 1;
   return cudaGetLastError();
 }

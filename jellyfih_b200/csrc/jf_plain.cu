@@ -406,7 +406,7 @@ cudaError_t jf_slots_out_launch(jf_engine* e, int m, float2* x, float2* v, float
                                 float* Jp, float* glow, float2* fiber) {
   const JfInst& I = e->inst[m];
   slots_out_kernel<<<blocks_for(I.n_slots), kThreads, 0, e->stream>>>(I, e->p, x, v, C, F, mat, Jp, glow, fiber,
-                                                                     e->h_slot_bad);
+                                                                     e->d_slot_bad);
   e->launches += 1;
   return cudaGetLastError();
 }
@@ -414,7 +414,7 @@ cudaError_t jf_slots_out_launch(jf_engine* e, int m, float2* x, float2* v, float
 cudaError_t jf_slots_in_launch(jf_engine* e, int m, const float2* x, const float2* v, const float4* C,
                                const float4* F, const float* Jp, const float* glow) {
   const JfInst& I = e->inst[m];
-  slots_in_kernel<<<blocks_for(I.n_slots), kThreads, 0, e->stream>>>(I, e->p, x, v, C, F, Jp, glow, e->h_slot_bad);
+  slots_in_kernel<<<blocks_for(I.n_slots), kThreads, 0, e->stream>>>(I, e->p, x, v, C, F, Jp, glow, e->d_slot_bad);
   e->launches += 1;
   return cudaGetLastError();
 }
